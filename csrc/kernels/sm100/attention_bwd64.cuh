@@ -232,14 +232,17 @@ flash_bwd64_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int g = base + it;
           if (it < n_iters) {
             if (!PROF_WAIT(t_q, mbar_wait(&q_full[g % ST], (g / ST) & 1, abort_flag, p.status, kStatusTimeoutFull))) { ok = false; break; }
-            // half a of the previous tile has been read out of tensor memory (across items the previous item's last
-            // tile was waited for through pds[1])
+            // half a of the previous tile has been read out of tensor memory (across items the products of the
+            // previous item's last tile have waited for both halves)
             if (it > 0 && !PROF_WAIT(t_pds0, mbar_wait(&pds[0], (g - 1) & 1, abort_flag, p.status, kStatusTimeoutTmemFull))) { ok = false; break; }
             tc_fence_after();
             scores(0, g % ST);
           }
           if (it > 0) {
             const int j = it - 1, gj = g - 1, sj = gj % ST, bq = gj & 1;
+            // the last tile of an item has no scores(0) of a next tile in front of its products, so its half a has not
+            // been waited for yet (the two compute groups run side by side: half b may be done first)
+            if (it == n_iters && !PROF_WAIT(t_pds0, mbar_wait(&pds[0], gj & 1, abort_flag, p.status, kStatusTimeoutTmemFull))) { ok = false; break; }
             if (!PROF_WAIT(t_pds1, mbar_wait(&pds[1], gj & 1, abort_flag, p.status, kStatusTimeoutTmemFull))) { ok = false; break; }
             if (gj >= 2 && !PROF_WAIT(t_dq, mbar_wait(&dq_drained[bq], ((gj >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutTmemEmpty))) {
               ok = false;
