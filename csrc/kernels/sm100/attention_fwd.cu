@@ -1,15 +1,23 @@
 // Causal online-softmax (flash) attention forward for sm_100a, GQA-aware.
 //
-// One CTA owns a 128-row query tile of one head.  K/V tiles stream in by TMA (local memory, no
-// multicast); S = Q K^T is a tcgen05.mma into tensor memory; 128 softmax threads (one query row
-// each, so row max / row sum need no shuffles) read S with tcgen05.ld, keep the running max and sum
-// in the log2 domain, write P as bf16 into 128B-swizzled shared memory, and a second tcgen05.mma
-// accumulates O += P V in tensor memory.  O is only rescaled when the running max grew by more than
-// 2^8 (the final division by the row sum makes the result exact either way), and the rescale is a
-// tcgen05.ld / tcgen05.st round trip over the 128 accumulator lanes.  Two CTAs fit per SM (96 KB
-// shared memory, 256 TMEM columns each) so one CTA's exponentials overlap the other's MMAs.  Inside a CTA the
-// next score product S_{j+1} is issued as soon as the softmax threads hold S_j in registers (barrier s_free), and
-// O += P_j V_j signals its own barrier (pv_done), so both products run under the softmax math of the next tile.
+// One persistent CTA per SM owns TWO 128-row query tiles of one head at a time.  Q and the K / V tiles (128 rows each, a
+// ring) come in by TMA (local memory, no multicast).  For query tile w: S_w = Q_w K^T is a tcgen05.mma into tensor
+// memory; 128 softmax threads (one query row each, so row max / row sum need no shuffles) read S_w, keep the running
+// max and sum in the log2 domain and write P_w as bf16 back over S_w's columns; O_w += P_w V takes P_w straight from
+// tensor memory.  While one tile's threads work on exponentials the tensor core runs the other tile's two products:
+//
+//   tensor core : S0(j) | PV1(j-1) S1(j) | PV0(j) S0(j+1) | PV1(j) S1(j+1) | ...
+//   softmax 0   :        P0(j)           |      ...       |   P0(j+1)
+//   softmax 1   :   ...  |    P1(j)                       |   ...
+//
+// O_w is only rescaled when the running max grew by more than 2^8 (the final division by the row sum makes the result
+// exact either way); the softmax threads do it themselves, with a tcgen05.ld / tcgen05.st round trip.
+//
+// What bounds it: per 128 x 128 scores at head_dim 128 the tensor core needs 1024 clocks and the exponentials also 1024
+// (16 a clock and SM); at head_dim 64 512 against 1024.  One query tile per CTA with P through shared memory, two CTAs
+// per SM (the split before this one), made P's round trip and the wait for its product part of every tile's chain:
+// B 8, H 32, T 4096, D 128: 1505 -> 941 us (731 -> 1169 TFLOP/s); B 1, H 24 / 8, T 8191, D 128: 485 -> 328 us;
+// B 4, H 32 / 4, T 2048, D 64: 137 -> 121 us; B 8, H 12, T 1024, D 64: 43 -> 38 us; one tile (T 61): 10 us both.
 //
 // The reference has no attention kernel in use: its CPU path materialises softmax(QK^T s + mask) V
 // (crates/incin-backends/src/cpu/ops/shape_ops.rs:1245-1269) and CUDA reports SDPA as unsupported;
@@ -24,86 +32,109 @@ namespace incin {
 int make_operand_map(CUtensorMap* out, const void* ptr, long long inner, long long rows, long long ld,
                      long long batch_lo, long long stride_lo, long long batch_hi, long long stride_hi, int box_inner,
                      int box_rows);
+int device_sm_count();
 
-constexpr int FA_BM = 128;
-constexpr int FA_THREADS = 192;
+constexpr int FA_BM = 128;        // rows of one query tile and of one K / V tile
+constexpr int FA_THREADS = 384;   // warp 0: TMA, warp 1: tcgen05 issue, warps 4-7 / 8-11: softmax of query tile 0 / 1
+// Registers: 384 threads are launched with 168 each (64512 of the SM's 65536).  The first warpgroup gives back all but 88
+// and the two softmax warpgroups take 208, enough to hold a whole row of scores: 128 x (88 + 208 + 208) = 64512.
+constexpr int FA_REGS_ISSUE = 88, FA_REGS_SOFTMAX = 208;
 
-template <int D, int BN>
+template <int D>
 struct FaCfg {
-  static constexpr int Q_BYTES = FA_BM * D * 2;
-  static constexpr int K_BYTES = BN * D * 2;
-  static constexpr int V_BYTES = BN * D * 2;
-  static constexpr int P_BYTES = FA_BM * BN * 2;
-  static constexpr int K_STAGES = 2;
-  static constexpr int OFF_K = Q_BYTES;
-  static constexpr int OFF_V = OFF_K + K_STAGES * K_BYTES;
-  static constexpr int OFF_P = OFF_V + V_BYTES;
-  static constexpr int OFF_BAR = OFF_P + P_BYTES;
+  static constexpr int TILE_BYTES = FA_BM * D * 2;      // one Q, K or V tile
+  static constexpr int STAGES = D == 128 ? 5 : 8;       // ring of K_0 V_0 K_1 V_1 ... tiles
+  static constexpr int OFF_RING = 2 * TILE_BYTES;       // behind the two query tiles
+  static constexpr int OFF_BAR = OFF_RING + STAGES * TILE_BYTES;
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
-  static constexpr int TMEM_COLS = 256;  // S: [0, BN), O: [BN, BN + D)
+  // tensor memory: S_w (P_w in its first 64 columns) at [128 w, 128 w + 128), O_w at 256 + D w
+  static constexpr int TMEM_COLS = 512, COL_O = 256;
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared-memory plan");
 };
 
 struct FaParams {
-  int T, Hq, Hkv, n_q_tiles;
+  int T, Hq, Hkv, B;
+  int n_pairs;       // pairs of query tiles per head
   float scale_log2;  // softmax scale * log2(e)
   __nv_bfloat16* O;
   long long o_stride_b, o_stride_t, o_stride_h;
   float* lse;  // [B, Hq, Tpad], log2 domain; rows in [T, Tpad) are written as +inf
   int Tpad;
   int* status;
-  int tile_major;   // 1: grid = (heads, batch, query tiles), else (query tiles, heads, batch)
+  int pair_major;   // 1: all heads' heaviest pairs come first in the item list, 0: the pairs of one head are neighbours
 };
 
-template <int D, int BN>
-__global__ void __launch_bounds__(FA_THREADS, 2)
+// a * b + c on two fp32 lanes at once (one issue slot)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+
+template <int D>
+__global__ void __launch_bounds__(FA_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const FaParams p) {
-  using Cfg = FaCfg<D, BN>;
+  using Cfg = FaCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = smem + Cfg::OFF_K;
-  uint8_t* sV = smem + Cfg::OFF_V;
-  uint8_t* sP = smem + Cfg::OFF_P;
+  uint8_t* sRing = smem + Cfg::OFF_RING;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::OFF_BAR);
-  uint64_t* q_full = bars;         // 1
-  uint64_t* k_full = bars + 1;     // [2]
-  uint64_t* k_empty = bars + 3;    // [2]
-  uint64_t* v_full = bars + 5;     // 1
-  uint64_t* v_empty = bars + 6;    // 1
-  uint64_t* s_full = bars + 7;     // 1: S_j is in tensor memory
-  uint64_t* p_full = bars + 8;     // one arrival per softmax warp: P_j in shared memory, O rescaled
-  uint64_t* s_free = bars + 9;     // one arrival per softmax warp: S_j has been read into registers
-  uint64_t* pv_done = bars + 10;   // 1: O += P_j V_j has finished (P_j's shared memory and O may be touched again)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint64_t* full = bars;            // [STAGES <= 8] a K or V tile has landed
+  uint64_t* empty = bars + 8;       // [STAGES <= 8] the products that read it have finished
+  uint64_t* q_full = bars + 16;     // [2] query tile w has landed
+  uint64_t* q_empty = bars + 18;    // [2] the last score product of query tile w has finished
+  uint64_t* s_full = bars + 20;     // [2] S_w is in tensor memory (and every earlier product has finished)
+  uint64_t* p_full = bars + 22;     // [2] P_w is in tensor memory, O_w rescaled (one arrival per softmax warp)
+  uint64_t* o_full = bars + 24;     // [2] O_w of this item is complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Blocks are dispatched x-fastest.  Heavy (late) query tiles go first either way.  When K / V of all heads together
-  // fit L2 (tile_major), the query tile is the slowest index: ALL heads' heaviest tiles start first and the light ones
-  // fill the gaps at the end (longest-processing-time order over the whole launch; GPT-2 layer 0.050 -> 0.038 ms).
-  // Otherwise a head's tiles stay together so that its K / V are read from DRAM once (with B 8, H 32, S 4096, D 128
-  // the global order cost 19 %).
-  const int q_tile = p.n_q_tiles - 1 - (int)(p.tile_major ? blockIdx.z : blockIdx.x);
-  const int hq = p.tile_major ? blockIdx.x : blockIdx.y, b = p.tile_major ? blockIdx.y : blockIdx.z;
-  const int hkv = hq / (p.Hq / p.Hkv);
-  const int q0 = q_tile * FA_BM;
-  int last_kv = q0 + FA_BM - 1;
-  if (last_kv > p.T - 1) last_kv = p.T - 1;
-  const int n_tiles = last_kv / BN + 1;
+  const int n_heads = p.Hq * p.B;
+  const int n_items = p.n_pairs * n_heads;
+  // Item list, walked in snake order (round r of CTA c: item r G + c, in odd rounds (r + 1) G - 1 - c), so that a CTA
+  // which got a long item in one round gets a short one in the next.  When K / V of all heads together fit L2
+  // (pair_major), the pair is the slowest index: all heads' heaviest pairs come first and the light ones fill the gaps
+  // at the end.  Otherwise a head's pairs are neighbours, so that its K / V are read from DRAM once.
+  auto item_of = [&](int r, int& q0, int& hq, int& b) -> bool {
+    const int G = (int)gridDim.x, c = (int)blockIdx.x;
+    const int idx = (r & 1) ? (r + 1) * G - 1 - c : r * G + c;
+    if (idx >= n_items) return false;
+    const int pair = p.pair_major ? idx / n_heads : idx % p.n_pairs;
+    const int hb = p.pair_major ? idx % n_heads : idx / p.n_pairs;
+    q0 = (p.n_pairs - 1 - pair) * (2 * FA_BM);
+    hq = hb % p.Hq;
+    b = hb / p.Hq;
+    return true;
+  };
+  // K / V tiles that query tile w of the item sees (causal); 0 when the tile lies beyond the sequence
+  auto kv_tiles = [&](int q0, int w) -> int {
+    const int first = q0 + w * FA_BM;
+    return first >= p.T ? 0 : min(first + FA_BM - 1, p.T - 1) / FA_BM + 1;
+  };
 
   if (threadIdx.x == 0) {
-    mbar_init(q_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
+    for (int s = 0; s < Cfg::STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
     }
-    mbar_init(v_full, 1);
-    mbar_init(v_empty, 1);
-    mbar_init(s_full, 1);
-    mbar_init(p_full, 4);   // one arrival per softmax warp
-    mbar_init(s_free, 4);
-    mbar_init(pv_done, 1);
+    for (int w = 0; w < 2; ++w) {
+      mbar_init(&q_full[w], 1);
+      mbar_init(&q_empty[w], 1);
+      mbar_init(&s_full[w], 1);
+      mbar_init(&p_full[w], 4);
+      mbar_init(&o_full[w], 1);
+    }
     *abort_flag = 0;
     mbar_init_fence();
     tma_prefetch_desc(&tmQ);
@@ -118,206 +149,242 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + BN;
   pdl_launch_dependents();   // tensor memory is held; a successor may be scheduled as CTAs retire
   pdl_wait();                // no global memory was touched above
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(FA_REGS_ISSUE));
   if (warp == 0) {
     // producer: the whole warp walks the loop (warp-uniform waits and address arithmetic), one elected lane issues
     const bool leader = elect_one() != 0;
-    {
-      if (leader) {
-        mbar_expect_tx(q_full, Cfg::Q_BYTES);
-#pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_4d(sQ + c * (FA_BM * 128), &tmQ, q_full, c * 64, q0, hq, b);
-      }
-      for (int j = 0; j < n_tiles; ++j) {
-        const int ks = j & 1;
-        if (!mbar_wait(&k_empty[ks], ((j >> 1) & 1) ^ 1, abort_flag, p.status, kStatusTimeoutEmpty)) break;
+    int stage = 0;
+    uint32_t phase = 0, q_phase[2] = {0, 0};
+    bool ok = true;
+    int q0, hq, b;
+    for (int r = 0; ok && item_of(r, q0, hq, b); ++r) {
+      const int hkv = hq / (p.Hq / p.Hkv);
+      const int n1 = kv_tiles(q0, 1), n = max(kv_tiles(q0, 0), n1);
+      auto load_q = [&](int w) -> bool {
+        if (!mbar_wait(&q_empty[w], q_phase[w] ^ 1, abort_flag, p.status, kStatusTimeoutEmpty)) return false;
+        q_phase[w] ^= 1;
         if (leader) {
-          mbar_expect_tx(&k_full[ks], Cfg::K_BYTES);
+          mbar_expect_tx(&q_full[w], Cfg::TILE_BYTES);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c)
-            tma_load_4d(sK + ks * Cfg::K_BYTES + c * (BN * 128), &tmK, &k_full[ks], c * 64, j * BN, hkv, b);
-        }
-        if (!mbar_wait(v_empty, (j & 1) ^ 1, abort_flag, p.status, kStatusTimeoutEmpty)) break;
-        if (leader) {
-          mbar_expect_tx(v_full, Cfg::V_BYTES);
-#pragma unroll
-          for (int c = 0; c < D / 64; ++c) tma_load_4d(sV + c * (BN * 128), &tmV, v_full, c * 64, j * BN, hkv, b);
-        }
-        __syncwarp();
-      }
-    }
-  } else if (warp == 1) {
-    // issuer: the whole warp walks the loop, one elected lane executes the tcgen05 instructions
-    const bool leader = elect_one() != 0;
-    {
-      constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, BN, false, false);
-      constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, D, false, true);
-      // S_{j+1} = Q K_{j+1}^T is issued as soon as the softmax threads have S_j in registers, so it and O += P_j V_j
-      // run while they work on the exponentials of tile j+1; the chain of a tile is then the softmax math alone.
-      auto issue_s = [&](int j) -> bool {
-        const int ks = j & 1;
-        if (!mbar_wait(&k_full[ks], (j >> 1) & 1, abort_flag, p.status, kStatusTimeoutFull)) return false;
-        if (j > 0 && !mbar_wait(s_free, (j - 1) & 1, abort_flag, p.status, kStatusTimeoutTmemEmpty)) return false;
-        tc_fence_after();
-        const uint32_t aq = smem_u32(sQ), bk = smem_u32(sK + ks * Cfg::K_BYTES);
-#pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint64_t ad = make_smem_desc(aq + (kk >> 2) * (FA_BM * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc(bk + (kk >> 2) * (BN * 128) + (kk & 3) * 32, 16, 1024);
-          if (leader) umma_f16_ss(tmem_S, ad, bd, idesc_s, kk > 0 ? 1u : 0u);
-        }
-        if (leader) {
-          umma_commit(&k_empty[ks]);
-          umma_commit(s_full);
+            tma_load_4d(smem + w * Cfg::TILE_BYTES + c * (FA_BM * 128), &tmQ, &q_full[w], c * 64, q0 + w * FA_BM, hq, b);
         }
         __syncwarp();
         return true;
       };
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.status, kStatusTimeoutFull);
-      ok = ok && issue_s(0);
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        if (j + 1 < n_tiles && !issue_s(j + 1)) { ok = false; break; }
-        if (!mbar_wait(p_full, j & 1, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
-        if (!mbar_wait(v_full, j & 1, abort_flag, p.status, kStatusTimeoutFull)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t ap = smem_u32(sP), bv = smem_u32(sV);
-#pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk) {
-          const uint64_t ad = make_smem_desc(ap + (kk >> 2) * (FA_BM * 128) + (kk & 3) * 32, 16, 1024);
-          const uint64_t bd = make_smem_desc(bv + kk * 2048, BN * 128, 1024);  // V^T: MN-major, 16 kv rows per step
-          if (leader) umma_f16_ss(tmem_O, ad, bd, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
-        }
+      auto load_kv = [&](const CUtensorMap* tm, int j) -> bool {
+        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, kStatusTimeoutEmpty)) return false;
         if (leader) {
-          umma_commit(v_empty);
-          umma_commit(pv_done);
+          mbar_expect_tx(&full[stage], Cfg::TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_4d(sRing + stage * Cfg::TILE_BYTES + c * (FA_BM * 128), tm, &full[stage], c * 64, j * FA_BM, hkv, b);
+        }
+        __syncwarp();
+        if (++stage == Cfg::STAGES) {
+          stage = 0;
+          phase ^= 1;
+        }
+        return true;
+      };
+      ok = load_q(0) && load_kv(&tmK, 0) && (n1 == 0 || load_q(1)) && load_kv(&tmV, 0);
+      for (int j = 1; j < n && ok; ++j) ok = load_kv(&tmK, j) && load_kv(&tmV, j);
+    }
+  } else if (warp == 1) {
+    // issuer: the whole warp walks the loop, one elected lane executes the tcgen05 instructions.  Products of one
+    // issuing thread run in order, so S_w(j+1) may follow O_w += P_w(j) V_j directly although it overwrites P_w.
+    const bool leader = elect_one() != 0;
+    constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BM, false, false);
+    constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, D, false, true);
+    constexpr uint32_t kDescHi = ((1024u >> 4) & 0x3FFF) | (1u << 14) | (2u << 29);   // SBO 1024, version, SWIZZLE_128B
+    constexpr uint32_t kLoK = (16u >> 4) << 16;                                       // K-major: LBO 16
+    constexpr uint32_t kLoMN = ((uint32_t)(FA_BM * 128) >> 4) << 16;                  // MN-major V: 64-column chunks 16 KB apart
+    auto desc = [&](uint32_t lo) -> uint64_t { return (static_cast<uint64_t>(kDescHi) << 32) | lo; };
+    const uint32_t q16 = (smem_u32(smem) & 0x3FFFF) >> 4, ring16 = (smem_u32(sRing) & 0x3FFFF) >> 4;
+    uint32_t q_phase[2] = {0, 0}, p_phase[2] = {0, 0};
+    int stage = 0;          // ring position of the next tile to be consumed
+    uint32_t phase = 0;
+    bool ok = true;
+    auto scores = [&](int w, int k_stage) {   // S_w = Q_w K^T
+      const uint32_t a = q16 + w * (Cfg::TILE_BYTES >> 4), bk = ring16 + k_stage * (Cfg::TILE_BYTES >> 4);
+#pragma unroll
+      for (int kk = 0; kk < D / 16; ++kk) {
+        const uint32_t off = (kk >> 2) * (FA_BM * 128 >> 4) + (kk & 3) * 2;
+        if (leader) umma_f16_ss(tmem_base + w * FA_BM, desc(a + off + kLoK), desc(bk + off + kLoK), idesc_s, kk > 0 ? 1u : 0u);
+      }
+      if (leader) umma_commit(&s_full[w]);
+      __syncwarp();
+    };
+    auto take = [&](int& my_stage) -> bool {   // next tile of the ring
+      if (!mbar_wait(&full[stage], phase, abort_flag, p.status, kStatusTimeoutFull)) return false;
+      my_stage = stage;
+      if (++stage == Cfg::STAGES) {
+        stage = 0;
+        phase ^= 1;
+      }
+      return true;
+    };
+    auto wait_q = [&](int w) -> bool {
+      if (!mbar_wait(&q_full[w], q_phase[w], abort_flag, p.status, kStatusTimeoutFull)) return false;
+      q_phase[w] ^= 1;
+      return true;
+    };
+    int q0, hq, b;
+    for (int r = 0; ok && item_of(r, q0, hq, b); ++r) {
+      const int n_w[2] = {kv_tiles(q0, 0), kv_tiles(q0, 1)};
+      const int n = max(n_w[0], n_w[1]);
+      int k_stage = 0, v_stage = 0;
+      ok = take(k_stage);
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        if (!ok || n_w[w] == 0) continue;
+        ok = wait_q(w);
+        if (!ok) continue;
+        tc_fence_after();
+        scores(w, k_stage);
+        if (leader && n_w[w] == 1) umma_commit(&q_empty[w]);
+      }
+      if (ok && leader) umma_commit(&empty[k_stage]);
+      for (int j = 0; j < n && ok; ++j) {
+        ok = take(v_stage);
+        if (ok && j + 1 < n) ok = take(k_stage);
+        if (!ok) break;
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+          if (!ok || j >= n_w[w]) continue;
+          ok = mbar_wait(&p_full[w], p_phase[w], abort_flag, p.status, kStatusTimeoutTmemFull);
+          if (!ok) continue;
+          p_phase[w] ^= 1;
+          tc_fence_after();
+          const uint32_t bv = ring16 + v_stage * (Cfg::TILE_BYTES >> 4);
+#pragma unroll
+          for (int kk = 0; kk < FA_BM / 16; ++kk)   // O_w += P_w V: 16 kv rows per product, P_w from tensor memory
+            if (leader) umma_f16_ts(tmem_base + Cfg::COL_O + w * D, tmem_base + w * FA_BM + kk * 8, desc(bv + kk * 128 + kLoMN),
+                                    idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          if (j + 1 < n_w[w]) {
+            scores(w, k_stage);
+            if (leader && j + 2 == n_w[w]) umma_commit(&q_empty[w]);
+          } else if (leader) {
+            umma_commit(&o_full[w]);
+          }
+          __syncwarp();
+        }
+        if (ok && leader) {
+          umma_commit(&empty[v_stage]);
+          if (j + 1 < n) umma_commit(&empty[k_stage]);
         }
         __syncwarp();
       }
     }
+  }
   } else {
-    // ------------------------------------------------------------------ softmax / correction / epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(FA_REGS_SOFTMAX));
+    // ------------------------------------------------------------------ softmax / rescale / epilogue of query tile w
+    const int w = (warp >> 2) - 1;
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;  // row inside the tile == TMEM lane
-    const int q_idx = q0 + row;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    float m_ref = -CUDART_INF_F, l_sum = 0.f;
+    const uint32_t tmem_S = tmem_base + w * FA_BM + lane_addr, tmem_O = tmem_base + Cfg::COL_O + w * D + lane_addr;
+    uint32_t s_phase = 0, o_phase = 0;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      if (!mbar_wait(s_full, j & 1, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
-      tc_fence_after();
-      const int kv0 = j * BN;
-      const bool need_mask = (kv0 + BN - 1 > q0) || (kv0 + BN > p.T);
-      // whole S row into registers with back-to-back TMEM loads and a single wait
-      uint32_t r[BN];
+    int q0, hq, b;
+    for (int r_item = 0; ok && item_of(r_item, q0, hq, b); ++r_item) {
+      const int n = kv_tiles(q0, w);
+      if (n == 0) continue;
+      const int q_idx = q0 + w * FA_BM + row;
+      float m_ref = -CUDART_INF_F;
+      float2 l2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      for (int j = 0; j < n; ++j) {
+        if (!mbar_wait(&s_full[w], s_phase, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
+        s_phase ^= 1;
+        tc_fence_after();
+        // whole S row into registers with back-to-back TMEM loads and a single wait
+        uint32_t s[FA_BM];
 #pragma unroll
-      for (int c = 0; c < BN / 32; ++c)
-        tmem_ld_32x32(tmem_S + lane_addr + c * 32, reinterpret_cast<uint32_t(&)[32]>(r[c * 32]));
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(s_free);   // the next score product may overwrite S
-      if (need_mask) {  // masked scores become -inf, so the code below needs no further tests
+        for (int c = 0; c < FA_BM / 32; ++c) tmem_ld_32x32(tmem_S + c * 32, reinterpret_cast<uint32_t(&)[32]>(s[c * 32]));
+        tmem_ld_wait();
+        if (j == n - 1) {   // the diagonal tile is the last one; masked scores become -inf
+          const int last = min(q_idx, p.T - 1) - j * FA_BM;
 #pragma unroll
-        for (int i = 0; i < BN; ++i) {
-          const int kv = kv0 + i;
-          if (!(kv <= q_idx && kv < p.T)) r[i] = __float_as_uint(-CUDART_INF_F);
+          for (int i = 0; i < FA_BM; ++i)
+            if (i > last) s[i] = __float_as_uint(-CUDART_INF_F);
         }
-      }
-      // row maximum with four independent chains
-      float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+        float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};   // four chains, three-input maxima
 #pragma unroll
-      for (int i = 0; i < BN; i += 4) {
-        mx4[0] = fmaxf(mx4[0], __uint_as_float(r[i]));
-        mx4[1] = fmaxf(mx4[1], __uint_as_float(r[i + 1]));
-        mx4[2] = fmaxf(mx4[2], __uint_as_float(r[i + 2]));
-        mx4[3] = fmaxf(mx4[3], __uint_as_float(r[i + 3]));
-      }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
-      // lazy rescale: only move the reference when the maximum grew by more than 2^8
-      const bool need = mx > m_ref + 8.0f;
-      float alpha = 1.0f;
-      if (need) {
-        alpha = exp2f(m_ref - mx);  // 0 on the first tile
-        m_ref = mx;
-        l_sum *= alpha;
-      }
-      // P = exp2(s * scale - m_ref) as packed bf16, kept in registers (in place of the scores they came from) while
-      // O += P_{j-1} V_{j-1} may still be running; four independent sum chains
-      const float neg_m = -m_ref;
-      float ls4[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int i = 0; i < FA_BM; i += 8)
 #pragma unroll
-      for (int i = 0; i < BN; i += 2) {
-        const float e0 = exp2f(fmaf(__uint_as_float(r[i]), p.scale_log2, neg_m));
-        const float e1 = exp2f(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, neg_m));
-        ls4[i & 3] += e0;
-        ls4[(i & 3) + 1] += e1;
-        r[i >> 1] = pack_bf16x2(e0, e1);
-      }
-      // that product must have finished before O is rescaled or P's shared memory is written again
-      if (j > 0 && !mbar_wait(pv_done, (j - 1) & 1, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
-      tc_fence_after();
-      if (j > 0 && __any_sync(0xffffffffu, need)) {
+          for (int e = 0; e < 4; ++e)
+            mx4[e] = fmaxf(fmaxf(mx4[e], __uint_as_float(s[i + e * 2])), __uint_as_float(s[i + e * 2 + 1]));
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+        // lazy rescale: only move the reference when the maximum grew by more than 2^8
+        const bool need = mx > m_ref + 8.0f;
+        if (__any_sync(0xffffffffu, need)) {
+          const float alpha = need ? exp2f(m_ref - mx) : 1.0f;   // 0 on the first tile
+          if (need) m_ref = mx;
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            l2[e].x *= alpha;
+            l2[e].y *= alpha;
+          }
+          if (j > 0) {   // s_full covers O_w += P_w(j-1) V_{j-1}: O_w is at rest
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_O + lane_addr + c * 32, o);
-          tmem_ld_wait();
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld_32x32(tmem_O + c * 32, o);
+              tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-          tmem_st_32x32(tmem_O + lane_addr + c * 32, o);
+              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st_32x32(tmem_O + c * 32, o);
+            }
+          }
+        }
+        // P = exp2(s * scale - m_ref) as packed bf16 over the first half of S_w's columns, row sums in fp32
+        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(-m_ref, -m_ref);
+#pragma unroll
+        for (int c = 0; c < FA_BM / 32; ++c) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = fma2(make_float2(__uint_as_float(s[c * 32 + i]), __uint_as_float(s[c * 32 + i + 1])), sc2, nm2);
+            const float2 e = make_float2(exp2f(x.x), exp2f(x.y));
+            l2[(i >> 1) & 1] = add2(l2[(i >> 1) & 1], e);
+            pk[i >> 1] = pack_bf16x2(e.x, e.y);
+          }
+          tmem_st_32x16(tmem_S + c * 16, pk);
         }
         tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();                        // every lane's stores and fences precede the single arrival of its warp
+        if (lane == 0) mbar_arrive(&p_full[w]);
       }
-      // P into 128B-swizzled shared memory: 16-byte unit ^ (row % 8)
-#pragma unroll
-      for (int c = 0; c < BN / 32; ++c) {
-        uint8_t* prow = sP + (c >> 1) * (FA_BM * 128) + row * 128;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int w0 = (c * 32 + u * 8) >> 1;
-          const int unit = ((c & 1) * 4 + u) ^ (row & 7);
-          *reinterpret_cast<uint4*>(prow + unit * 16) = make_uint4(r[w0], r[w0 + 1], r[w0 + 2], r[w0 + 3]);
-        }
-      }
-      l_sum += (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
-      fence_proxy_async_smem();
-      tc_fence_before();
-      __syncwarp();                        // every lane's writes and fences precede the single arrival of its warp
-      if (lane == 0) mbar_arrive(p_full);
-    }
-    if (ok && mbar_wait(pv_done, (n_tiles - 1) & 1, abort_flag, p.status, kStatusTimeoutTmemFull)) {
+      if (!ok || !mbar_wait(&o_full[w], o_phase, abort_flag, p.status, kStatusTimeoutTmemFull)) { ok = false; break; }
+      o_phase ^= 1;
       tc_fence_after();
+      const float l_sum = (l2[0].x + l2[0].y) + (l2[1].x + l2[1].y);
       const float inv = 1.0f / l_sum;
       const bool live_row = q_idx < p.T;
       __nv_bfloat16* orow = p.O + (long long)b * p.o_stride_b + (long long)q_idx * p.o_stride_t +
                             (long long)hq * p.o_stride_h;
+      const bool wide = aligned32(orow);
 #pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_O + lane_addr + c * 32, r);
+        uint32_t o[32];
+        tmem_ld_32x32(tmem_O + c * 32, o);
         tmem_ld_wait();
-        if (live_row && aligned32(orow)) {   // 32 bytes per store: whole sectors of the row
+        uint32_t pk[16];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            uint32_t o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-              o[e] = pack_bf16x2(__uint_as_float(r[u * 16 + e * 2]) * inv, __uint_as_float(r[u * 16 + e * 2 + 1]) * inv);
-            st_global_b256(orow + c * 32 + u * 16, o);
-          }
+        for (int e = 0; e < 16; ++e) pk[e] = pack_bf16x2(__uint_as_float(o[e * 2]) * inv, __uint_as_float(o[e * 2 + 1]) * inv);
+        if (live_row && wide) {   // 32 bytes per store: whole sectors of the row
+          st_global_b256(orow + c * 32, reinterpret_cast<uint32_t(&)[8]>(pk[0]));
+          st_global_b256(orow + c * 32 + 16, reinterpret_cast<uint32_t(&)[8]>(pk[8]));
         } else if (live_row) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            uint4 o;
-            o.x = pack_bf16x2(__uint_as_float(r[u * 8 + 0]) * inv, __uint_as_float(r[u * 8 + 1]) * inv);
-            o.y = pack_bf16x2(__uint_as_float(r[u * 8 + 2]) * inv, __uint_as_float(r[u * 8 + 3]) * inv);
-            o.z = pack_bf16x2(__uint_as_float(r[u * 8 + 4]) * inv, __uint_as_float(r[u * 8 + 5]) * inv);
-            o.w = pack_bf16x2(__uint_as_float(r[u * 8 + 6]) * inv, __uint_as_float(r[u * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = o;
-          }
+          for (int u = 0; u < 4; ++u)
+            *reinterpret_cast<uint4*>(orow + c * 32 + u * 8) = make_uint4(pk[u * 4], pk[u * 4 + 1], pk[u * 4 + 2], pk[u * 4 + 3]);
         }
         __syncwarp();
       }
@@ -336,35 +403,40 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
-template <int D, int BN>
+template <int D>
 static int launch_fwd(const incin_attn_desc* d, cudaStream_t stream) {
-  using Cfg = FaCfg<D, BN>;
+  using Cfg = FaCfg<D>;
   CUtensorMap tq, tk, tv;
   int rc = make_operand_map(&tq, d->q, D, d->T, d->q_stride_t, d->Hq, d->q_stride_h, d->B, d->q_stride_b, 64, FA_BM);
   if (rc) return rc;
-  rc = make_operand_map(&tk, d->k, D, d->T, d->k_stride_t, d->Hkv, d->k_stride_h, d->B, d->k_stride_b, 64, BN);
+  rc = make_operand_map(&tk, d->k, D, d->T, d->k_stride_t, d->Hkv, d->k_stride_h, d->B, d->k_stride_b, 64, FA_BM);
   if (rc) return rc;
-  rc = make_operand_map(&tv, d->v, D, d->T, d->v_stride_t, d->Hkv, d->v_stride_h, d->B, d->v_stride_b, 64, BN);
+  rc = make_operand_map(&tv, d->v, D, d->T, d->v_stride_t, d->Hkv, d->v_stride_h, d->B, d->v_stride_b, 64, FA_BM);
   if (rc) return rc;
-  auto kern = flash_fwd_kernel<D, BN>;
+  auto kern = flash_fwd_kernel<D>;
   static PerDeviceFlags attr;
   if (!ensure_dynamic_smem(kern, Cfg::SMEM_BYTES, attr)) return INCIN_ERR_LAUNCH;
+  const int n_q_tiles = (d->T + FA_BM - 1) / FA_BM;
   FaParams p;
   p.T = d->T;
   p.Hq = d->Hq;
   p.Hkv = d->Hkv;
-  p.n_q_tiles = (d->T + FA_BM - 1) / FA_BM;
+  p.B = d->B;
+  p.n_pairs = (n_q_tiles + 1) / 2;
   p.scale_log2 = d->scale * 1.4426950408889634f;
   p.O = (__nv_bfloat16*)d->o;
   p.o_stride_b = d->o_stride_b;
   p.o_stride_t = d->o_stride_t;
   p.o_stride_h = d->o_stride_h;
   p.lse = d->lse;
-  p.Tpad = p.n_q_tiles * FA_BM;
+  p.Tpad = n_q_tiles * FA_BM;
   p.status = (int*)d->status;
   // K and V of every (batch, kv head) against half of the 126 MB L2
-  p.tile_major = ((long long)d->B * d->Hkv * d->T * D * 2 * 2 <= (48ll << 20)) ? 1 : 0;
-  dim3 grid = p.tile_major ? dim3(d->Hq, d->B, p.n_q_tiles) : dim3(p.n_q_tiles, d->Hq, d->B);
+  p.pair_major = ((long long)d->B * d->Hkv * d->T * D * 2 * 2 <= (48ll << 20)) ? 1 : 0;
+  const long long items = (long long)p.n_pairs * d->Hq * d->B;
+  if (items > (1ll << 30)) return INCIN_ERR_TOO_LARGE;   // the kernel counts items in 32 bits
+  const int sms = device_sm_count();
+  const dim3 grid((unsigned)(items < sms ? items : sms));
   if (launch_pdl<true>(kern, grid, dim3(FA_THREADS), Cfg::SMEM_BYTES, stream, tq, tk, tv, p) != cudaSuccess) return INCIN_ERR_LAUNCH;
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
@@ -377,7 +449,7 @@ extern "C" int incin_flash_attn_fwd(const incin_attn_desc* d, void* stream) {
     return INCIN_ERR_ARGUMENT;
   if ((d->o_stride_t % 8) || (d->o_stride_h % 8) || (d->o_stride_b % 8) || (reinterpret_cast<uintptr_t>(d->o) & 15))
     return INCIN_ERR_ALIGNMENT;
-  if (d->D == 64) return incin::launch_fwd<64, 128>(d, (cudaStream_t)stream);
-  if (d->D == 128) return incin::launch_fwd<128, 64>(d, (cudaStream_t)stream);
+  if (d->D == 64) return incin::launch_fwd<64>(d, (cudaStream_t)stream);
+  if (d->D == 128) return incin::launch_fwd<128>(d, (cudaStream_t)stream);
   return INCIN_ERR_UNSUPPORTED;
 }

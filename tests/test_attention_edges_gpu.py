@@ -22,3 +22,30 @@ def test_backward_repeats_to_the_bit(B, T, H, D):
             first = (dk, dv)
         assert torch.equal(dk, first[0]) and torch.equal(dv, first[1])
     G.check_status()
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 1, 1), (2, 127, 3, 1), (1, 129, 2, 2), (3, 255, 2, 1), (1, 257, 4, 2),
+                                        (40, 384, 6, 2), (2, 1025, 5, 5)])
+def test_forward_tile_edges(B, T, Hq, Hkv, D):
+    """Query tiles come in pairs and items outnumber CTAs in some of these: one row, one tile, a pair with one tile
+    beyond the sequence, several items per CTA; strided inputs; rows whose scores need rescaling on every tile."""
+    from incin_b200.ops import attention as A
+    from incin_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(T + D)
+    x = torch.randn(B, T, Hq + 2 * Hkv, D, generator=g)
+    # keys grow along the sequence so that the running maximum moves by more than the rescale threshold
+    x[:, :, Hq:Hq + Hkv] *= torch.linspace(0.2, 6.0, T).view(1, T, 1, 1)
+    x = x.to(torch.bfloat16).cuda()
+    q, k, v = x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:]
+    with torch.no_grad():
+        out = A.flash_attention(q, k, v)
+    G.check_status()
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double().repeat_interleave(Hq // Hkv, 2)) * D ** -0.5
+    s = s.masked_fill(~torch.ones(T, T, device="cuda", dtype=torch.bool).tril(), float("-inf"))
+    p, vd = torch.softmax(s, -1), v.double().repeat_interleave(Hq // Hkv, 2)
+    ref = torch.einsum("bhqk,bkhd->bqhd", p, vd)
+    # bf16 keeps 8 bits, so rounding P costs up to 2^-8 of each term and rounding the output 2^-8 more:
+    # |error| <= 2^-8 (sum p |v| + |o|), 5 % above it for the fp32 scores, exponentials and sums
+    bound = 2.0 ** -8 * 1.05 * (torch.einsum("bhqk,bkhd->bqhd", p, vd.abs()) + ref.abs()) + 1e-5
+    assert ((out.double() - ref).abs() <= bound).all()
