@@ -14,7 +14,9 @@
 // exact either way); the softmax threads do it themselves, with a tcgen05.ld / tcgen05.st round trip.
 //
 // What bounds it: per 128 x 128 scores at head_dim 128 the tensor core needs 1024 clocks and the exponentials also 1024
-// (16 a clock and SM); at head_dim 64 512 against 1024.  One query tile per CTA with P through shared memory, two CTAs
+// (16 a clock and SM); at head_dim 64 512 against 1024.  Both units run at about 63 % (ncu): a tile's chain of loading, maximum,
+// exponentials and its two products is what is left over.  (2^x on the FMA pipe for a quarter of the scores changed
+// nothing, for more of them it was slower.)  One query tile per CTA with P through shared memory, two CTAs
 // per SM (the split before this one), made P's round trip and the wait for its product part of every tile's chain:
 // B 8, H 32, T 4096, D 128: 1505 -> 941 us (731 -> 1169 TFLOP/s); B 1, H 24 / 8, T 8191, D 128: 485 -> 328 us;
 // B 4, H 32 / 4, T 2048, D 64: 137 -> 121 us; B 8, H 12, T 1024, D 64: 43 -> 38 us; one tile (T 61): 10 us both.
@@ -49,6 +51,9 @@ struct FaCfg {
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
   // tensor memory: S_w (P_w in its first 64 columns) at [128 w, 128 w + 128), O_w at 256 + D w
   static constexpr int TMEM_COLS = 512, COL_O = 256;
+  // columns of P_w after which the first products of O_w += P_w V are let go: 96 of 128 takes 5 % off head_dim 128 (B 1,
+  // H 24 / 8, T 8191: 351 -> 335 us) and 3 % off head_dim 64 (B 4, H 32 / 4, T 2048: 122 -> 118 us); 64 is no better
+  static constexpr int PART = 96;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared-memory plan");
 };
 
@@ -96,7 +101,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* s_full = bars + 20;     // [2] S_w is in tensor memory (and every earlier product has finished)
   uint64_t* p_full = bars + 22;     // [2] P_w is in tensor memory, O_w rescaled (one arrival per softmax warp)
   uint64_t* o_full = bars + 24;     // [2] O_w of this item is complete
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+  uint64_t* p_part = bars + 26;     // [2] the first PART columns of P_w are in tensor memory, O_w rescaled
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -134,6 +140,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&s_full[w], 1);
       mbar_init(&p_full[w], 4);
       mbar_init(&o_full[w], 1);
+      mbar_init(&p_part[w], 4);
     }
     *abort_flag = 0;
     mbar_init_fence();
@@ -256,15 +263,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
         for (int w = 0; w < 2; ++w) {
           if (!ok || j >= n_w[w]) continue;
-          ok = mbar_wait(&p_full[w], p_phase[w], abort_flag, p.status, kStatusTimeoutTmemFull);
-          if (!ok) continue;
-          p_phase[w] ^= 1;
-          tc_fence_after();
           const uint32_t bv = ring16 + v_stage * (Cfg::TILE_BYTES >> 4);
+          // O_w += P_w V: 16 kv rows per product, P_w from tensor memory, the first products before all of P_w is there
+          ok = mbar_wait(&p_part[w], p_phase[w], abort_flag, p.status, kStatusTimeoutTmemFull);
+          if (!ok) continue;
+          tc_fence_after();
 #pragma unroll
-          for (int kk = 0; kk < FA_BM / 16; ++kk)   // O_w += P_w V: 16 kv rows per product, P_w from tensor memory
+          for (int kk = 0; kk < FA_BM / 16; ++kk) {
+            if (kk == Cfg::PART / 16) {
+              ok = mbar_wait(&p_full[w], p_phase[w], abort_flag, p.status, kStatusTimeoutTmemFull);
+              if (!ok) break;
+              tc_fence_after();
+            }
             if (leader) umma_f16_ts(tmem_base + Cfg::COL_O + w * D, tmem_base + w * FA_BM + kk * 8, desc(bv + kk * 128 + kLoMN),
                                     idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          }
+          if (!ok) continue;
+          p_phase[w] ^= 1;
           if (j + 1 < n_w[w]) {
             scores(w, k_stage);
             if (leader && j + 2 == n_w[w]) umma_commit(&q_empty[w]);
@@ -355,6 +370,12 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             pk[i >> 1] = pack_bf16x2(e.x, e.y);
           }
           tmem_st_32x16(tmem_S + c * 16, pk);
+          if ((c + 1) * 32 == Cfg::PART) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_part[w]);
+          }
         }
         tmem_st_wait();
         tc_fence_before();
