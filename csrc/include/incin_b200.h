@@ -57,7 +57,7 @@ typedef struct incin_gemm_desc {
   int out_fp32;    /* C is float instead of bf16 */
   int accumulate;  /* fp32 only: C += result (atomic), needed for split-K */
   float alpha;
-  const void* bias;     /* bf16 [N] or NULL */
+  const void* bias;     /* bf16 (or the operands' type, see in_dtype) [N], or NULL */
   const void* residual; /* bf16, same layout as C, or NULL */
   int act;
   void* aux;     /* bf16, same layout as C: GELU/SILU pre-activation out, DGELU/DSILU pre-activation in */
@@ -93,8 +93,9 @@ typedef struct incin_gemm_desc {
   long long rs_slot_stride;
   void* rs_ready;
   /* --- operand type: INCIN_GEMM_IN_BF16 (0), INCIN_GEMM_IN_FP16 or INCIN_GEMM_IN_TF32 (A and B are fp32, multiplied
-   * as tf32; K-contiguous operands only, lda / ldb multiples of 4).  The last two require out_fp32 and take no fused
-   * epilogue (bias, residual, activation), no CTA-pair tile and no fused collective. */
+   * as tf32; K-contiguous operands only, lda / ldb multiples of 4).  The last two take a bias of the operands' own type
+   * (not with accumulate), no other fused epilogue (residual, activation), no CTA-pair tile and no fused collective;
+   * out_fp32 == 0 writes fp16 for fp16 operands and is refused for tf32. */
   int in_dtype;
   /* --- optional device scalar (fp32) multiplied into alpha when the epilogue runs: lets a gradient that only exists
    * on the GPU (the upstream gradient of a loss) scale a product without a launch of its own. */
@@ -162,6 +163,8 @@ int incin_causal_softmax_bwd(void* dp, const void* p, long long batch, int T, fl
 /* ---- reductions / misc ------------------------------------------------------------------------- */
 /* dbias[n] += sum_m dy[m][n]  (fp32 accumulate into the flat gradient buffer) */
 int incin_colsum_accum(const void* dy, float* dbias, long long rows, int N, long long ld, void* stream);
+/* the same with dy of type INCIN_GEMM_IN_BF16, _FP16 or _TF32 (= fp32); the sums are fp32 */
+int incin_colsum_accum_typed(const void* dy, float* dbias, long long rows, int N, long long ld, int dtype, void* stream);
 /* out[0] += sum(x^2); out[1] = 1.0 if any element is NaN/Inf (device-side gradient check, no D2H of tensors) */
 int incin_sumsq_nonfinite_f32(const float* x, long long n, float* out, void* stream);
 int incin_fill_f32(float* x, float value, long long n, void* stream);
@@ -248,6 +251,8 @@ int incin_cumsum(const void* x, void* out, long long outer, long long n, long lo
  * (0 = broadcast): transpose, narrow, paste, broadcast, concat and pad are all this one copy. */
 int incin_strided_copy(const void* src, void* dst, int rank, const long long* shape, const long long* src_strides,
                        const long long* dst_strides, int elem_bytes, void* stream);
+/* dst[cols][rows] = src[rows][cols] (both dense); colsum, if not NULL: colsum[c] += sum_r src[r][c] */
+int incin_transpose_f32(const float* src, float* dst, long long rows, long long cols, float* colsum, void* stream);
 /* Indexed ops check every index: an out-of-range one is skipped and *err_flag (device int, may be NULL) is set. */
 int incin_gather_rows(const void* src, const long long* index, void* out, long long n_idx, long long row_elems,
                       long long src_rows, int elem_bytes, int* err_flag, void* stream);

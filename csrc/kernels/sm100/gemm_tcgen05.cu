@@ -511,7 +511,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         tmem_ld_32x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * Cfg::ACC_STRIDE + c * 32, r);
         tmem_ld_wait();
         const int nc = n0 + c * 32;
-        if (row_ok && nc < p.N) epilogue_chunk(p, r, c_ptr, cbase, nc, vec_ok, alpha);
+        if (row_ok && nc < p.N) {
+          if (p.in_kind == 0 || p.accumulate) epilogue_chunk(p, r, c_ptr, cbase, nc, vec_ok, alpha);
+          else epilogue_chunk_other(p, r, c_ptr, cbase, nc, alpha);
+        }
         __syncwarp();  // tcgen05.ld is warp-collective: reconverge before the next chunk
       }
       }
@@ -779,11 +782,13 @@ extern "C" int incin_gemm_bf16(const incin_gemm_desc* d, void* stream_) {
   // Other operand types.  fp16 changes only the format field of the instruction.  fp32 operands are multiplied as
   // tf32: a row of fp32 is moved by the same tensor maps as a row of twice as many 2-byte units (the 128-byte swizzle
   // works on 16-byte chunks), so from here on K and the operand strides count 2-byte units; only the instruction kind
-  // differs (8 fp32 = the same 32 bytes per product).  Both write fp32 and take no fused epilogue or collective.
+  // differs (8 fp32 = the same 32 bytes per product).  Both write fp32, fp16 operands also fp16, with at most a bias of
+  // the operands' type in the epilogue; no activation, residual or collective.
   incin_gemm_desc widened;
   const int in_kind = d->in_dtype;
   if (in_kind != INCIN_GEMM_IN_BF16) {
-    if ((in_kind != INCIN_GEMM_IN_FP16 && in_kind != INCIN_GEMM_IN_TF32) || !d->out_fp32 || d->bias || d->residual ||
+    if ((in_kind != INCIN_GEMM_IN_FP16 && in_kind != INCIN_GEMM_IN_TF32) ||
+        (!d->out_fp32 && (in_kind == INCIN_GEMM_IN_TF32 || d->accumulate)) || (d->bias && d->accumulate) || d->residual ||
         d->aux || d->act != INCIN_ACT_NONE || d->ag_world > 1 || d->rs_world > 1 || d->tile_n == 512)
       return INCIN_ERR_ARGUMENT;
     if (in_kind == INCIN_GEMM_IN_TF32) {
@@ -929,7 +934,8 @@ extern "C" int incin_gemm_bf16(const incin_gemm_desc* d, void* stream_) {
   CUtensorMap tc = ta, tx = ta;
   p.tma_out = 0;
   const bool short_k = (kb_total + splits - 1) / splits <= 16;
-  if (tma_out_on && !p.rs_world && d->C && (short_k || bn == 256 || tma_out_all)) {
+  const bool own_epilogue = in_kind != INCIN_GEMM_IN_BF16 && (d->bias || !d->out_fp32);   // not staged
+  if (tma_out_on && !own_epilogue && !p.rs_world && d->C && (short_k || bn == 256 || tma_out_all)) {
     if (d->out_fp32) {
       p.tma_out = (!with_pre && make_f32_reduce_map(&tc, d->C, d->N, d->M, d->ldc, blo, d->c_stride_lo, bhi, d->c_stride_hi, 32) == INCIN_OK) ? 1 : 0;
     } else {   // bf16 rows leave with 16-byte stores: C (and the side output) 16-byte aligned with strides in multiples of 8

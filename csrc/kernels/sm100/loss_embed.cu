@@ -8,6 +8,7 @@
 #include "ptx.cuh"
 #include "launch.cuh"
 #include "../../include/incin_b200.h"
+#include <cuda_fp16.h>
 #include <math_constants.h>
 
 namespace incin {
@@ -287,10 +288,14 @@ causal_softmax_bwd_kernel(__nv_bfloat16* __restrict__ dp, const __nv_bfloat16* _
 }
 
 // ----------------------------------------------------------------------------- column sum (bias gradient)
+__device__ __forceinline__ float to_f32(float v) { return v; }
+__device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
+__device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
+
 // block = 32 x 8 threads covering 64 columns; grid.y row chunks; fp32 atomics into the gradient buffer
+template <typename T>
 __global__ void __launch_bounds__(256)
-colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dbias, long long rows, int N, long long ld,
-              int chunks) {
+colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long rows, int N, long long ld, int chunks) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float sh[8][64];
@@ -301,15 +306,16 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dbias, l
   const long long r1 = r0 + rows_per < rows ? r0 + rows_per : rows;
   float a0 = 0.f, a1 = 0.f;
   if (c0 < N) {
-    const bool pair = (c0 + 1 < N) && ((ld & 1) == 0);
+    struct alignas(2 * sizeof(T)) Pair { T x, y; };
+    const bool pair = (c0 + 1 < N) && ((ld & 1) == 0) && (reinterpret_cast<uintptr_t>(dy) % sizeof(Pair)) == 0;
     for (long long r = r0 + ty; r < r1; r += 8) {
       if (pair) {
-        const float2 v = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(dy + r * ld + c0));
-        a0 += v.x;
-        a1 += v.y;
+        const Pair v = *reinterpret_cast<const Pair*>(dy + r * ld + c0);
+        a0 += to_f32(v.x);
+        a1 += to_f32(v.y);
       } else {
-        a0 += __bfloat162float(dy[r * ld + c0]);
-        if (c0 + 1 < N) a1 += __bfloat162float(dy[r * ld + c0 + 1]);
+        a0 += to_f32(dy[r * ld + c0]);
+        if (c0 + 1 < N) a1 += to_f32(dy[r * ld + c0 + 1]);
       }
     }
   }
@@ -329,41 +335,59 @@ colsum_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dbias, l
   }
 }
 
-// 16-byte variant: 32 lanes x 8 columns = 256 columns per block, 8 row lanes, needs N % 8 == 0 and ld % 8 == 0
+// 16-byte variant: 32 lanes x VEC columns (8 of 16 bits, 4 fp32) per block, 8 row lanes; needs N % VEC == 0 and
+// ld % VEC == 0
+template <typename T>
 __global__ void __launch_bounds__(256)
-colsum_vec_kernel(const __nv_bfloat16* __restrict__ dy, float* __restrict__ dbias, long long rows, int N,
-                  long long ld, int chunks) {
+colsum_vec_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long rows, int N, long long ld, int chunks) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float sh[8][256];
+  constexpr int VEC = 16 / sizeof(T);
+  __shared__ float sh[8][32 * VEC];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * 256 + tx * 8;
+  const int c0 = blockIdx.x * (32 * VEC) + tx * VEC;
   const long long rows_per = (rows + chunks - 1) / chunks;
   const long long r0 = (long long)blockIdx.y * rows_per;
   const long long r1 = r0 + rows_per < rows ? r0 + rows_per : rows;
-  float a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  float a[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; ++i) a[i] = 0.f;
   if (c0 < N) {
     for (long long r = r0 + ty; r < r1; r += 8) {
       const uint4 u = *reinterpret_cast<const uint4*>(dy + r * ld + c0);
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+      const T* e = reinterpret_cast<const T*>(&u);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = unpack_bf16x2(w[i]);
-        a[2 * i] += f.x;
-        a[2 * i + 1] += f.y;
-      }
+      for (int i = 0; i < VEC; ++i) a[i] += to_f32(e[i]);
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) sh[ty][tx * 8 + i] = a[i];
+  for (int i = 0; i < VEC; ++i) sh[ty][tx * VEC + i] = a[i];
   __syncthreads();
-  const int c = blockIdx.x * 256 + threadIdx.x;
-  if (c < N) {
+  const int c = blockIdx.x * (32 * VEC) + threadIdx.x;
+  if (threadIdx.x < 32 * VEC && c < N) {
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
     atomicAdd(dbias + c, t);
   }
+}
+
+template <typename T>
+static int colsum_launch(const void* dy, float* dbias, long long rows, int N, long long ld, cudaStream_t stream) {
+  constexpr int VEC = 16 / sizeof(T);
+  cudaError_t e;
+  if ((N % VEC) == 0 && (ld % VEC) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0) {
+    const int colblocks = (N + 32 * VEC - 1) / (32 * VEC);
+    long long chunks = (148 * 4 + colblocks - 1) / colblocks;
+    if (chunks > (rows + 31) / 32) chunks = (rows + 31) / 32;
+    if (chunks < 1) chunks = 1;
+    e = launch_pdl(colsum_vec_kernel<T>, dim3(colblocks, (unsigned)chunks), dim3(256), 0, stream, (const T*)dy, dbias, rows, N, ld, (int)chunks);
+  } else {
+    long long chunks = (rows + 255) / 256;
+    if (chunks > 128) chunks = 128;
+    e = launch_pdl(colsum_kernel<T>, dim3((N + 63) / 64, (unsigned)chunks), dim3(256), 0, stream, (const T*)dy, dbias, rows, N, ld, (int)chunks);
+  }
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
 }  // namespace incin
@@ -437,19 +461,14 @@ extern "C" int incin_causal_softmax_bwd(void* dp, const void* p, long long batch
 }
 
 extern "C" int incin_colsum_accum(const void* dy, float* dbias, long long rows, int N, long long ld, void* stream) {
+  return incin_colsum_accum_typed(dy, dbias, rows, N, ld, INCIN_GEMM_IN_BF16, stream);
+}
+
+extern "C" int incin_colsum_accum_typed(const void* dy, float* dbias, long long rows, int N, long long ld, int dtype, void* stream) {
   if (rows <= 0 || N <= 0) return INCIN_ERR_ARGUMENT;
-  if ((N % 8) == 0 && (ld % 8) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0) {
-    const int colblocks = (N + 255) / 256;
-    long long chunks = (148 * 4 + colblocks - 1) / colblocks;
-    if (chunks > (rows + 31) / 32) chunks = (rows + 31) / 32;
-    if (chunks < 1) chunks = 1;
-    dim3 grid(colblocks, (unsigned)chunks);
-    launch_pdl(colsum_vec_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)dy, dbias, rows, N, ld, (int)chunks);
-    return CHECK_LAUNCH();
-  }
-  long long chunks = (rows + 255) / 256;
-  if (chunks > 128) chunks = 128;
-  dim3 grid((N + 63) / 64, (unsigned)chunks);
-  launch_pdl(colsum_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const __nv_bfloat16*)dy, dbias, rows, N, ld, (int)chunks);
-  return CHECK_LAUNCH();
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == INCIN_GEMM_IN_BF16) return colsum_launch<__nv_bfloat16>(dy, dbias, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_FP16) return colsum_launch<__half>(dy, dbias, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_TF32) return colsum_launch<float>(dy, dbias, rows, N, ld, s);
+  return INCIN_ERR_ARGUMENT;
 }

@@ -58,22 +58,65 @@ __global__ void strided_copy_vec_kernel(const T* __restrict__ src, T* __restrict
   }
 }
 
-// 2-D transpose of the two innermost axes through a padded shared tile (outer axes batched in blockIdx.z)
-template <typename T>
-__global__ void transpose_tile_kernel(const T* __restrict__ src, T* __restrict__ dst, long long rows, long long cols,
-                                      long long s_batch, long long d_batch) {
-  __shared__ T tile[32][33];
+// 2-D transpose of the two innermost axes through a padded 64 x 64 shared tile (outer axes batched in blockIdx.z).  Bound
+// by memory: with VEC both sides move 16 bytes a thread (rows and columns multiples of 16 bytes, aligned bases); 32 x 32
+// tiles of single elements reached half of that.  COLSUM (float only) adds the column sums of the source to colsum on
+// the way, which saves the bias gradient its own pass over the matrix.
+template <typename T, bool VEC, bool COLSUM>
+__global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict__ src, T* __restrict__ dst, long long rows,
+                                                             long long cols, long long s_batch, long long d_batch,
+                                                             float* __restrict__ colsum) {
+  constexpr int V = VEC ? 16 / (int)sizeof(T) : 1;   // elements per access
+  constexpr int TPR = 64 / V;                        // threads per row of the tile
+  constexpr int PITCH = sizeof(T) == 2 ? 66 : 65;    // 2-byte rows start 33 words apart: no bank conflicts on the way in
+  __shared__ T tile[64 * PITCH];
   const T* s = src + blockIdx.z * s_batch;
   T* d = dst + blockIdx.z * d_batch;
-  const long long c0 = (long long)blockIdx.x * 32, r0 = (long long)blockIdx.y * 32;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const long long r = r0 + j, c = c0 + threadIdx.x;
-    if (r < rows && c < cols) tile[j][threadIdx.x] = s[r * cols + c];
+  const long long c0 = (long long)blockIdx.x * 64, r0 = (long long)blockIdx.y * 64;
+  const int tv = (threadIdx.x % TPR) * V, tr = threadIdx.x / TPR;
+  float sum[V];
+  if constexpr (COLSUM) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) sum[k] = 0.f;
+  }
+#pragma unroll
+  for (int j = tr; j < 64; j += 256 / TPR) {
+    const long long r = r0 + j, c = c0 + tv;
+    if (r < rows && c < cols) {
+      alignas(16) T e[V];
+      if constexpr (VEC) *reinterpret_cast<uint4*>(e) = *reinterpret_cast<const uint4*>(s + r * cols + c);
+      else e[0] = s[r * cols + c];
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        tile[j * PITCH + tv + k] = e[k];
+        if constexpr (COLSUM) sum[k] += (float)e[k];
+      }
+    }
   }
   __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const long long c = c0 + j, r = r0 + threadIdx.x;
-    if (r < rows && c < cols) d[c * rows + r] = tile[threadIdx.x][j];
+#pragma unroll
+  for (int j = tr; j < 64; j += 256 / TPR) {
+    const long long c = c0 + j, r = r0 + tv;
+    if (r < rows && c < cols) {
+      alignas(16) T e[V];
+#pragma unroll
+      for (int k = 0; k < V; ++k) e[k] = tile[(tv + k) * PITCH + j];
+      if constexpr (VEC) *reinterpret_cast<uint4*>(d + c * rows + r) = *reinterpret_cast<const uint4*>(e);
+      else d[c * rows + r] = e[0];
+    }
+  }
+  if constexpr (COLSUM) {
+    __syncthreads();
+    float* part = reinterpret_cast<float*>(tile);    // [256 / TPR][64]
+#pragma unroll
+    for (int k = 0; k < V; ++k) part[tr * 64 + tv + k] = sum[k];
+    __syncthreads();
+    if (threadIdx.x < 64 && c0 + threadIdx.x < cols) {
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < 256 / TPR; ++k) t += part[k * 64 + threadIdx.x];
+      atomicAdd(colsum + c0 + threadIdx.x, t);
+    }
   }
 }
 
@@ -175,6 +218,17 @@ inline unsigned grid_for(long long n, int block) {
   return (unsigned)(g < 1 ? 1 : (g > 148LL * 16 ? 148LL * 16 : g));
 }
 
+// src [batch, rows, cols] -> dst [batch, cols, rows], both dense; at most 65535 batches and 65535 x 64 rows
+template <typename T, bool COLSUM>
+int transpose_launch(const T* src, T* dst, long long rows, long long cols, long long batch, float* colsum, cudaStream_t s) {
+  constexpr int V = 16 / sizeof(T);
+  const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64), (unsigned)batch);
+  const bool vec = rows % V == 0 && cols % V == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+  if (vec) transpose_tile_kernel<T, true, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
+  else transpose_tile_kernel<T, false, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
+  return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
+}
+
 template <typename T>
 int strided_copy_t(const void* src, void* dst, const Geometry& g, cudaStream_t s) {
   long long total = 1;
@@ -187,11 +241,8 @@ int strided_copy_t(const void* src, void* dst, const Geometry& g, cudaStream_t s
       g.sstride[last - 1] == 1 && g.sstride[last] == g.shape[last - 1]) {
     const long long rows = g.shape[last], cols = g.shape[last - 1];   // source is [.., rows(last), cols(last-1)] dense
     const long long batch = g.rank == 3 ? g.shape[0] : 1;
-    if (batch <= 65535 && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols))) {
-      dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32), (unsigned)batch), block(32, 8);
-      transpose_tile_kernel<T><<<grid, block, 0, s>>>(static_cast<const T*>(src), static_cast<T*>(dst), rows, cols, rows * cols,
-                                                      rows * cols);
-      return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
+    if (batch <= 65535 && (rows + 63) / 64 <= 65535 && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols))) {
+      return transpose_launch<T, false>(static_cast<const T*>(src), static_cast<T*>(dst), rows, cols, batch, nullptr, s);
     }
   }
   bool vec = g.sstride[last] == 1 && g.dstride[last] == 1 && g.shape[last] % VEC == 0 &&
@@ -227,6 +278,14 @@ extern "C" int incin_strided_copy(const void* src, void* dst, int rank, const lo
     case 8: return strided_copy_t<unsigned long long>(src, dst, g, s);
     default: return INCIN_ERR_ARGUMENT;
   }
+}
+
+extern "C" int incin_transpose_f32(const float* src, float* dst, long long rows, long long cols, float* colsum, void* stream) {
+  if (!src || !dst || rows <= 0 || cols <= 0) return INCIN_ERR_ARGUMENT;
+  if ((rows + 63) / 64 > 65535) return INCIN_ERR_TOO_LARGE;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return colsum ? transpose_launch<float, true>(src, dst, rows, cols, 1, colsum, s)
+                : transpose_launch<float, false>(src, dst, rows, cols, 1, nullptr, s);
 }
 
 extern "C" int incin_gather_rows(const void* src, const long long* index, void* out, long long n_idx, long long row_elems,

@@ -66,10 +66,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, M: int, N: int,
     dst: [ptr]*world, slot_stride} makes the epilogue store partial tiles into the owners' slot buffers."""
     assert a.dtype == b.dtype and a.dtype in _IN_KIND, "operands must both be bf16, fp16 or fp32 (multiplied as tf32)"
     in_kind = _IN_KIND[a.dtype]
-    assert out.dtype in (torch.bfloat16, torch.float32)
-    if in_kind != nat.GEMM_IN_BF16:
-        # fp16 / tf32 operands: fp32 output, no fused epilogue; tf32 wants K-contiguous operands
-        assert out.dtype == torch.float32 and bias is None and residual is None and aux is None and act == nat.ACT_NONE
+    if in_kind == nat.GEMM_IN_BF16:
+        assert out.dtype in (torch.bfloat16, torch.float32)
+    else:
+        # fp16 / tf32 operands: output fp32 or the operands' type, no fused epilogue but a bias of the operands' type;
+        # tf32 wants K-contiguous operands
+        assert out.dtype in (torch.float32, a.dtype) and residual is None and aux is None and act == nat.ACT_NONE
+        assert bias is None or (bias.dtype == a.dtype and not accumulate)
         assert gather is None and scatter is None and tile_n != 512
         assert in_kind == nat.GEMM_IN_FP16 or not (a_mn or b_mn)
     if tile_n == 0 and not accumulate and gather is None and scatter is None and in_kind == nat.GEMM_IN_BF16:
@@ -159,7 +162,7 @@ def mm_nt(x: torch.Tensor, w: torch.Tensor, *, bias=None, residual=None, act=nat
 
 
 def mm_nt_f32out(x: torch.Tensor, w: torch.Tensor, *, alpha: float = 1.0, out: torch.Tensor | None = None,
-                 accumulate: bool = False) -> torch.Tensor:
+                 accumulate: bool = False, splits: int = 1) -> torch.Tensor:
     """fp32 y[..., N] = x[..., K] @ w[N, K]^T on the tensor cores for bf16, fp16 or fp32 operands (fp32 operands are
     multiplied as tf32: 10 mantissa bits per factor, fp32 accumulation).  K must be a multiple of 8 (16-bit types)
     or 4 (fp32) so that every row starts on a 16-byte boundary."""
@@ -168,7 +171,16 @@ def mm_nt_f32out(x: torch.Tensor, w: torch.Tensor, *, alpha: float = 1.0, out: t
     N = w.shape[0]
     if out is None:
         out = torch.empty(*x.shape[:-1], N, dtype=torch.float32, device=x.device)
-    return gemm(x, w, out, M=M, N=N, K=K, lda=K, ldb=K, ldc=N, alpha=alpha, accumulate=accumulate)
+    return gemm(x, w, out, M=M, N=N, K=K, lda=K, ldb=K, ldc=N, alpha=alpha, accumulate=accumulate, splits=splits)
+
+
+def mm_linear_other(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
+    """y[M, N] = x[M, K] @ w[N, K]^T + bias for fp16 or fp32 (multiplied as tf32) operands, in the operands' type: fp32
+    accumulation, one rounding."""
+    M, K = x.shape
+    N = w.shape[0]
+    out = torch.empty(M, N, dtype=x.dtype, device=x.device)
+    return gemm(x, w, out, M=M, N=N, K=K, lda=K, ldb=K, ldc=N, bias=bias)
 
 
 def mm_nn(dy: torch.Tensor, w: torch.Tensor, *, act=nat.ACT_NONE, aux=None, out: torch.Tensor | None = None,

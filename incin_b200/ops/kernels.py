@@ -143,10 +143,23 @@ def causal_softmax_bwd_(dp, p, T, scale):
     return dp
 
 
+_COLSUM_KIND = {torch.bfloat16: nat.GEMM_IN_BF16, torch.float16: nat.GEMM_IN_FP16, torch.float32: nat.GEMM_IN_TF32}
+
+
 def colsum_accum(dy, dbias):
+    """``dbias[n] += sum_m dy[m, n]`` in fp32 for bf16, fp16 or fp32 ``dy``."""
     N = dy.shape[-1]
     rows = dy.numel() // N
-    nat.check(nat.cuda().incin_colsum_accum(dy.data_ptr(), dbias.data_ptr(), rows, N, N, _s()), "colsum")
+    nat.check(nat.cuda().incin_colsum_accum_typed(dy.data_ptr(), dbias.data_ptr(), rows, N, N, _COLSUM_KIND[dy.dtype], _s()),
+              "colsum")
+
+
+def transpose_f32(x, colsum=None):
+    """Dense transpose of a dense fp32 matrix; ``colsum`` (fp32), if given, gets the column sums of ``x`` added."""
+    rows, cols = x.shape
+    out = torch.empty(cols, rows, dtype=F32, device=x.device)
+    nat.check(nat.cuda().incin_transpose_f32(x.data_ptr(), out.data_ptr(), rows, cols, nat.ptr(colsum), _s()), "transpose_f32")
+    return out
 
 
 def sumsq_nonfinite(x, out):

@@ -1,0 +1,44 @@
+"""Linear in fp16 and fp32 (multiplied as tf32): epilogue with bias, transposed operands, column sums."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,n_in,n_out", [(1, 8, 8), (7, 24, 40), (64, 256, 64), (130, 264, 1000), (200, 72, 12),
+                                             (515, 64, 36), (1028, 768, 200), (96, 40, 33)])
+def test_linear_forward_backward(dtype, rows, n_in, n_out):
+    """Against 64 bits; every route of the backward is reached (n_out or rows no multiple of 16 bytes, ragged tiles)."""
+    from incin_b200.core.policy import MathMode, policy_scope
+    from incin_b200.ops import functional as F
+    from incin_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(rows + n_out)
+    x, w, b, dy = (torch.randn(*s, generator=g).to(dtype).cuda() for s in ((rows, n_in), (n_out, n_in), (n_out,), (rows, n_out)))
+    x, w, b = (t.requires_grad_() for t in (x, w, b))
+    with policy_scope(math=MathMode.FAST):
+        y = F.linear(x, w, b)
+        dx, dw, db = torch.autograd.grad(y, (x, w, b), dy)
+    G.check_status()
+    xd, wd, bd, dyd = (t.detach().double() for t in (x, w, b, dy))
+    # fp16: one rounding of the result (2^-11) and fp32 sums.  tf32: factors cut to 11 bits, 2^-10 each at worst.
+    u = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -9
+    for got, a, c, extra in ((y, xd, wd.t(), bd), (dx, dyd, wd, None), (dw, dyd.t(), xd, None)):
+        ref = a @ c + (0 if extra is None else extra)
+        bound = u * ref.abs() + (2.0 ** -20 if dtype == torch.float16 else u) * (a.abs() @ c.abs()) + 1e-6
+        assert ((got.double() - ref).abs() <= bound).all()
+    bound = 2.0 ** -11 * dyd.sum(0).abs() + 2.0 ** -20 * dyd.abs().sum(0)
+    assert ((db.double() - dyd.sum(0)).abs() <= bound + 1e-6).all() and db.dtype == dtype
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
+@pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48)])
+def test_transpose_tiles(dtype, batch, rows, cols):
+    from incin_b200.ops import tensor_ops as T
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randint(0, 255, (batch, rows, cols), generator=g).to(dtype).cuda()
+    assert torch.equal(T.materialize(x.transpose(1, 2)), x.transpose(1, 2).contiguous())
+    flat = torch.zeros(batch * rows * cols + 1, dtype=dtype, device="cuda")   # a base that is not 16-byte aligned
+    flat[1:] = x.reshape(-1)
+    odd = flat[1:].view(batch, rows, cols)
+    assert torch.equal(T.materialize(odd.transpose(1, 2)), x.transpose(1, 2).contiguous())
