@@ -41,12 +41,24 @@ def _ok_view(t: torch.Tensor) -> bool:
             and t.data_ptr() % 16 == 0 and t.dtype == torch.bfloat16)
 
 
-def _set(d: AttnDesc, name: str, t: torch.Tensor) -> None:
-    setattr(d, name if name != "do" else "d_o", t.data_ptr())
-    sb, st, sh, _ = t.stride()
-    setattr(d, f"{name}_stride_b", sb)
-    setattr(d, f"{name}_stride_t", st)
-    setattr(d, f"{name}_stride_h", sh)
+def _desc(q, k, v, o, lse, scale) -> AttnDesc:
+    """Descriptor of a forward call (one constructor call in field order; see the GEMM's)."""
+    B, T, Hq, D = q.shape
+    d = AttnDesc(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, T, Hq, k.shape[2], D, scale,
+                 *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3])
+    d.status = status_word(q.device).data_ptr()
+    return d
+
+
+def _run_bwd(q, k, v, o, lse, scale, do, dq, dk, dv) -> None:
+    B, T, Hq, D = q.shape
+    delta = torch.empty_like(lse)
+    acc = torch.empty(B, T, Hq, D, dtype=torch.float32, device=q.device)
+    d = AttnDesc(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), B, T, Hq, k.shape[2], D, scale,
+                 *q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3], do.data_ptr(), *do.stride()[:3],
+                 dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), *dq.stride()[:3], *dk.stride()[:3], *dv.stride()[:3],
+                 delta.data_ptr(), acc.data_ptr(), status_word(q.device).data_ptr())
+    nat.check(nat.cuda().incin_flash_attn_bwd(C.byref(d), nat.stream_ptr()), "flash_attn_bwd")
 
 
 def flash_shape_supported(T: int, head_dim: int, hq: int, hkv: int) -> bool:
@@ -60,11 +72,7 @@ class _Flash(torch.autograd.Function):
         Hkv = k.shape[2]
         o = torch.empty(B, T, Hq, D, dtype=torch.bfloat16, device=q.device)
         lse = torch.empty(B, Hq, (T + 127) // 128 * 128, dtype=torch.float32, device=q.device)
-        d = AttnDesc()
-        d.B, d.T, d.Hq, d.Hkv, d.D, d.scale = B, T, Hq, Hkv, D, scale
-        _set(d, "q", q), _set(d, "k", k), _set(d, "v", v), _set(d, "o", o)
-        d.lse = lse.data_ptr()
-        d.status = status_word(q.device).data_ptr()
+        d = _desc(q, k, v, o, lse, scale)
         nat.check(nat.cuda().incin_flash_attn_fwd(C.byref(d), nat.stream_ptr()), "flash_attn_fwd")
         ctx.save_for_backward(q, k, v, o, lse)
         ctx.scale = scale
@@ -81,15 +89,7 @@ class _Flash(torch.autograd.Function):
         # gets a single contiguous gradient back through autograd's view backward with no concatenation
         packed = torch.empty(B, T, Hq + 2 * Hkv, D, dtype=torch.bfloat16, device=q.device)
         dq, dk, dv = packed[:, :, :Hq], packed[:, :, Hq:Hq + Hkv], packed[:, :, Hq + Hkv:]
-        delta = torch.empty_like(lse)
-        acc = torch.empty(B, T, Hq, D, dtype=torch.float32, device=q.device)
-        d = AttnDesc()
-        d.B, d.T, d.Hq, d.Hkv, d.D, d.scale = B, T, Hq, Hkv, D, ctx.scale
-        _set(d, "q", q), _set(d, "k", k), _set(d, "v", v), _set(d, "o", o), _set(d, "do", do)
-        _set(d, "dq", dq), _set(d, "dk", dk), _set(d, "dv", dv)
-        d.lse, d.delta, d.dq_accum = lse.data_ptr(), delta.data_ptr(), acc.data_ptr()
-        d.status = status_word(q.device).data_ptr()
-        nat.check(nat.cuda().incin_flash_attn_bwd(C.byref(d), nat.stream_ptr()), "flash_attn_bwd")
+        _run_bwd(q, k, v, o, lse, ctx.scale, do, dq, dk, dv)
         return dq, dk, dv, None
 
 
@@ -105,20 +105,19 @@ class _FlashPacked(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, Hq, Hkv, D, scale):
-        B, T, _ = qkv.shape
-        x = qkv.view(B, T, Hq + 2 * Hkv, D)
-        q, k, v = x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:]
-        o = torch.empty(B, T, Hq, D, dtype=torch.bfloat16, device=qkv.device)
+        B, T, width = qkv.shape
+        o = torch.empty(B, T, Hq * D, dtype=torch.bfloat16, device=qkv.device)
         lse = torch.empty(B, Hq, (T + 127) // 128 * 128, dtype=torch.float32, device=qkv.device)
-        d = AttnDesc()
-        d.B, d.T, d.Hq, d.Hkv, d.D, d.scale = B, T, Hq, Hkv, D, scale
-        _set(d, "q", q), _set(d, "k", k), _set(d, "v", v), _set(d, "o", o)
-        d.lse = lse.data_ptr()
+        # q, k and v are column ranges of the packed rows: addresses and strides without building the views
+        at = qkv.data_ptr()
+        strides = (T * width, width, D)
+        d = AttnDesc(at, at + 2 * Hq * D, at + 2 * (Hq + Hkv) * D, o.data_ptr(), lse.data_ptr(), B, T, Hq, Hkv, D, scale,
+                     *strides, *strides, *strides, T * Hq * D, Hq * D, D)
         d.status = status_word(qkv.device).data_ptr()
         nat.check(nat.cuda().incin_flash_attn_fwd(C.byref(d), nat.stream_ptr()), "flash_attn_fwd")
         ctx.save_for_backward(qkv, o, lse)
         ctx.dims = (Hq, Hkv, D, scale)
-        return o.view(B, T, Hq * D)
+        return o
 
     @staticmethod
     def backward(ctx, do):
@@ -128,17 +127,10 @@ class _FlashPacked(torch.autograd.Function):
         do = do.contiguous().view(B, T, Hq, D)
         x = qkv.view(B, T, Hq + 2 * Hkv, D)
         q, k, v = x[:, :, :Hq], x[:, :, Hq:Hq + Hkv], x[:, :, Hq + Hkv:]
+        o = o.view(B, T, Hq, D)
         dqkv = torch.empty_like(x)
         dq, dk, dv = dqkv[:, :, :Hq], dqkv[:, :, Hq:Hq + Hkv], dqkv[:, :, Hq + Hkv:]
-        delta = torch.empty_like(lse)
-        acc = torch.empty(B, T, Hq, D, dtype=torch.float32, device=qkv.device)
-        d = AttnDesc()
-        d.B, d.T, d.Hq, d.Hkv, d.D, d.scale = B, T, Hq, Hkv, D, scale
-        _set(d, "q", q), _set(d, "k", k), _set(d, "v", v), _set(d, "o", o), _set(d, "do", do)
-        _set(d, "dq", dq), _set(d, "dk", dk), _set(d, "dv", dv)
-        d.lse, d.delta, d.dq_accum = lse.data_ptr(), delta.data_ptr(), acc.data_ptr()
-        d.status = status_word(qkv.device).data_ptr()
-        nat.check(nat.cuda().incin_flash_attn_bwd(C.byref(d), nat.stream_ptr()), "flash_attn_bwd")
+        _run_bwd(q, k, v, o, lse, scale, do, dq, dk, dv)
         return dqkv.view(B, T, -1), None, None, None, None
 
 

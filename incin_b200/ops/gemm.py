@@ -75,34 +75,21 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, M: int, N: int,
         assert bias is None or (bias.dtype == a.dtype and not accumulate)
         assert gather is None and scatter is None and tile_n != 512
         assert in_kind == nat.GEMM_IN_FP16 or not (a_mn or b_mn)
-    if tile_n == 0 and not accumulate and gather is None and scatter is None and in_kind == nat.GEMM_IN_BF16:
+    if (tile_n == 0 and not accumulate and gather is None and scatter is None and in_kind == nat.GEMM_IN_BF16
+            and _tuning_on()):
         tile_n = _tuned_tile_n(locals())
-    d = nat.GemmDesc()
+    # one positional constructor call in field order: setting two dozen fields by name costs several times as much, and
+    # short sequences are bound by what a launch costs on the host
+    d = nat.GemmDesc(a.data_ptr() + a.element_size() * a_offset, b.data_ptr() + b.element_size() * b_offset,
+                     out.data_ptr() + out.element_size() * c_offset, M, N, K, lda, ldb, ldc, a_mn, b_mn, batch[0], batch[1],
+                     a_strides[0], a_strides[1], b_strides[0], b_strides[1], c_strides[0], c_strides[1],
+                     out.dtype == torch.float32, accumulate, alpha, bias.data_ptr() if bias is not None else None,
+                     residual.data_ptr() if residual is not None else None, act, aux.data_ptr() if aux is not None else None,
+                     splits, tile_n, max_ctas, status_word(a.device).data_ptr())
     d.in_dtype = in_kind
-    d.A = a.data_ptr() + a.element_size() * a_offset
-    d.B = b.data_ptr() + b.element_size() * b_offset
-    d.C = out.data_ptr() + out.element_size() * c_offset
-    d.M, d.N, d.K = M, N, K
-    d.lda, d.ldb, d.ldc = lda, ldb, ldc
-    d.a_mn_major, d.b_mn_major = int(a_mn), int(b_mn)
-    d.batch_lo, d.batch_hi = batch
-    d.a_stride_lo, d.a_stride_hi = a_strides
-    d.b_stride_lo, d.b_stride_hi = b_strides
-    d.c_stride_lo, d.c_stride_hi = c_strides
-    d.out_fp32 = int(out.dtype == torch.float32)
-    d.accumulate = int(accumulate)
-    d.alpha = alpha
     if alpha_dev is not None:   # fp32 device scalar multiplied into alpha by the epilogue
         assert alpha_dev.dtype == torch.float32 and alpha_dev.numel() == 1 and alpha_dev.is_cuda
         d.alpha_ptr = alpha_dev.data_ptr()
-    d.bias = nat.ptr(bias)
-    d.residual = nat.ptr(residual)
-    d.act = act
-    d.aux = nat.ptr(aux)
-    d.splits = splits
-    d.tile_n = tile_n
-    d.max_ctas = max_ctas
-    d.status = status_word(a.device).data_ptr()
     if gather is not None:
         d.ag_world, d.ag_rank, d.ag_rows_per_rank = gather["world"], gather["rank"], gather["rows_per_rank"]
         d.ag_copy_ctas = gather.get("copy_ctas", 8)
@@ -123,14 +110,25 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, M: int, N: int,
 _IN_KIND = {torch.bfloat16: nat.GEMM_IN_BF16, torch.float16: nat.GEMM_IN_FP16, torch.float32: nat.GEMM_IN_TF32}
 
 
+_tuning = None
+
+
+def _tuning_on() -> bool:
+    """False with the default policy and nothing cached: the kernel library's own choice of tile stands."""
+    global _tuning
+    if _tuning is None:
+        from .. import tuning
+        _tuning = tuning
+    svc = _tuning.service()
+    return bool(svc.lru) or svc.policy not in (_tuning.TuningPolicy.DISABLED, _tuning.TuningPolicy.HEURISTIC)
+
+
 def _tuned_tile_n(kw: dict) -> int:
     """Ask the autotune service for the N tile of this problem.  With the default policy this is a dictionary
     lookup that falls through to the kernel's own heuristic (0); under ``coordinated_warmup`` /
     ``profile_guided`` the tile widths (512 = the CTA-pair tile) are timed once per (shape, layout) and the winner is cached."""
-    from ..tuning import TuningPolicy, candidates, service, time_cuda
+    from ..tuning import candidates, service, time_cuda
     svc = service()
-    if svc.policy in (TuningPolicy.DISABLED, TuningPolicy.HEURISTIC) and not svc.lru:
-        return 0
     key = (f"gemm/{kw['M']}x{kw['N']}x{kw['K']}/{int(kw['a_mn'])}{int(kw['b_mn'])}/b{kw['batch'][0] * kw['batch'][1]}"
            f"/e{kw['act']}{int(kw['bias'] is not None)}{int(kw['residual'] is not None)}")
     if torch.cuda.is_current_stream_capturing():   # nothing can be timed inside a capture: use what warm-up found
