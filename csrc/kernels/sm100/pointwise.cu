@@ -166,39 +166,85 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_
     dx[i] = __float2bfloat16(__bfloat162float(dy[i]) * act_grad(__bfloat162float(pre[i]), act));
 }
 
-// gate_up: [rows][2F] with gate = [:, :F], up = [:, F:]
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long long rows,
-                                  int F) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const long long total = rows * F;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const long long r = i / F;
-    const int c = (int)(i - r * F);
-    const float g = __bfloat162float(gu[r * 2 * F + c]);
-    const float u = __bfloat162float(gu[r * 2 * F + F + c]);
-    y[i] = __float2bfloat16(silu(g) * u);
+// gate_up: [rows][2F] with gate = [:, :F], up = [:, F:].  Bound by memory (6 bytes an element forward, 10 backward).  VEC:
+// eight elements a thread, 16 bytes an access (F a multiple of 8, aligned bases); one element a thread with a 64-bit
+// division each reached a third of the bandwidth.  8192 rows, F 5632, bf16: forward 139 -> 44 us, backward
+// 164 -> 75 us.
+template <bool VEC>
+__device__ __forceinline__ void ld_bf16(const __nv_bfloat16* p, float (&v)[VEC ? 8 : 1]) {
+  if constexpr (VEC) {
+    const uint4 u = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = unpack_bf16x2(w[i]);
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+    }
+  } else {
+    v[0] = __bfloat162float(p[0]);
   }
 }
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
-                                  __nv_bfloat16* __restrict__ dgu, long long rows, int F) {
+template <bool VEC>
+__device__ __forceinline__ void st_bf16(__nv_bfloat16* p, const float (&v)[VEC ? 8 : 1]) {
+  if constexpr (VEC)
+    *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+  else p[0] = __float2bfloat16(v[0]);
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(256) swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ y, long long rows,
+                                                         int F) {
   pdl_launch_dependents();
   pdl_wait();
-  const long long total = rows * F;
-  const long long stride = (long long)gridDim.x * blockDim.x;
+  constexpr int V = VEC ? 8 : 1;
+  const int per_row = F / V;
+  const long long total = rows * per_row, stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const long long r = i / F;
-    const int c = (int)(i - r * F);
-    const float g = __bfloat162float(gu[r * 2 * F + c]);
-    const float u = __bfloat162float(gu[r * 2 * F + F + c]);
-    const float d = __bfloat162float(dy[i]);
-    dgu[r * 2 * F + c] = __float2bfloat16(d * u * silu_grad(g));
-    dgu[r * 2 * F + F + c] = __float2bfloat16(d * silu(g));
+    const long long r = total <= 0xffffffffLL ? (long long)((unsigned)i / (unsigned)per_row) : i / per_row;
+    const __nv_bfloat16* p = gu + r * 2 * F + (i - r * per_row) * V;
+    float g[V], u[V];
+    ld_bf16<VEC>(p, g);
+    ld_bf16<VEC>(p + F, u);
+#pragma unroll
+    for (int k = 0; k < V; ++k) g[k] = silu(g[k]) * u[k];
+    st_bf16<VEC>(y + i * V, g);
+  }
+}
+template <bool VEC>
+__global__ void __launch_bounds__(256) swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ gu,
+                                                         __nv_bfloat16* __restrict__ dgu, long long rows, int F) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int V = VEC ? 8 : 1;
+  const int per_row = F / V;
+  const long long total = rows * per_row, stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const long long r = total <= 0xffffffffLL ? (long long)((unsigned)i / (unsigned)per_row) : i / per_row;
+    const long long o = r * 2 * F + (i - r * per_row) * V;
+    float g[V], u[V], d[V];
+    ld_bf16<VEC>(gu + o, g);
+    ld_bf16<VEC>(gu + o + F, u);
+    ld_bf16<VEC>(dy + i * V, d);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const float dg = d[k] * u[k] * silu_grad(g[k]);
+      u[k] = d[k] * silu(g[k]);
+      g[k] = dg;
+    }
+    st_bf16<VEC>(dgu + o, g);
+    st_bf16<VEC>(dgu + o + F, u);
   }
 }
 
 // Rotary embedding, "rotate-half" convention: pairs (i, i + D/2), angle = t * theta^(-2i/D).
+__device__ __forceinline__ float2 rope_angle(int t, int d, int D, float theta, int inverse) {   // (cos, sin)
+  const float freq = powf(theta, -2.f * d / D);
+  float sn, cs;
+  sincosf(t * freq, &sn, &cs);
+  return make_float2(cs, inverse ? -sn : sn);
+}
+
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long B, int T, int H, int D, long long sb,
                             long long st, long long sh, float theta, int inverse) {
   pdl_launch_dependents();
@@ -214,13 +260,47 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long B, int T, i
     const int t = (int)(r % T);
     const long long b = r / T;
     __nv_bfloat16* p = x + b * sb + (long long)t * st + (long long)h * sh;
-    const float freq = powf(theta, -2.f * d / D);
-    float sn, cs;
-    sincosf(t * freq, &sn, &cs);
-    if (inverse) sn = -sn;
+    const float2 cs = rope_angle(t, d, D, theta, inverse);
     const float a = __bfloat162float(p[d]), c = __bfloat162float(p[d + half]);
-    p[d] = __float2bfloat16(a * cs - c * sn);
-    p[d + half] = __float2bfloat16(c * cs + a * sn);
+    p[d] = __float2bfloat16(a * cs.x - c * cs.y);
+    p[d + half] = __float2bfloat16(c * cs.x + a * cs.y);
+  }
+}
+
+// The same for 16-byte aligned rows with D / 2 a multiple of 8 (at most ROPE_MAX_HALF).  A block takes ROPE_TOKENS
+// positions, works out their angles once for all heads (power, sine and cosine per pair and head were most of the general
+// kernel's time) and rotates eight pairs a thread with 16-byte accesses.  Bound by memory; 8192 positions, 36 heads of 64:
+// 57 -> 16 us.
+constexpr int ROPE_TOKENS = 8, ROPE_MAX_HALF = 128;
+__global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long positions, int T, int H, int D, long long sb,
+                                                       long long st, long long sh, float theta, int inverse) {
+  pdl_launch_dependents();
+  __shared__ float2 angle[ROPE_TOKENS * ROPE_MAX_HALF];
+  const int half = D / 2, vecs = half / 8;
+  const long long first = (long long)blockIdx.x * ROPE_TOKENS;
+  const int n = (int)(positions - first < ROPE_TOKENS ? positions - first : ROPE_TOKENS);
+  for (int i = threadIdx.x; i < n * half; i += 256)
+    angle[i] = rope_angle((int)((first + i / half) % T), i % half, D, theta, inverse);
+  __syncthreads();
+  pdl_wait();
+  const int per = H * vecs;
+  for (int i = threadIdx.x; i < n * per; i += 256) {
+    const int tok = i / per, k = i - tok * per, h = k / vecs, v = k - h * vecs;
+    const long long pos = first + tok, b = pos / T;
+    __nv_bfloat16* p = x + b * sb + (pos - b * T) * st + (long long)h * sh + v * 8;
+    float a[8], c[8];
+    ld_bf16<true>(p, a);
+    ld_bf16<true>(p + half, c);
+    const float2* cs = angle + tok * half + v * 8;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float2 q = cs[e];
+      const float r = a[e] * q.x - c[e] * q.y;
+      c[e] = c[e] * q.x + a[e] * q.y;
+      a[e] = r;
+    }
+    st_bf16<true>(p, a);
+    st_bf16<true>(p + half, c);
   }
 }
 
@@ -347,24 +427,35 @@ extern "C" int incin_act_bwd(const void* dy, const void* pre, void* dx, long lon
                                                            (__nv_bfloat16*)dx, n, act);
   return CHECK_LAUNCH();
 }
+static bool vec16(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
 extern "C" int incin_swiglu_fwd(const void* gate_up, void* y, long long rows, int F, void* stream) {
   if (rows <= 0 || F <= 0) return INCIN_ERR_ARGUMENT;
-  launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * F, 256)), dim3(256), 0, ST(stream), (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)y,
-                                                                     rows, F);
+  const bool vec = F % 8 == 0 && vec16(gate_up, y, y);
+  launch_pdl(vec ? swiglu_fwd_kernel<true> : swiglu_fwd_kernel<false>, dim3(grid_for(rows * (vec ? F / 8 : F), 256)), dim3(256), 0, ST(stream),
+             (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)y, rows, F);
   return CHECK_LAUNCH();
 }
 extern "C" int incin_swiglu_bwd(const void* dy, const void* gate_up, void* dgate_up, long long rows, int F,
                                 void* stream) {
   if (rows <= 0 || F <= 0) return INCIN_ERR_ARGUMENT;
-  launch_pdl(swiglu_bwd_kernel, dim3(grid_for(rows * F, 256)), dim3(256), 0, ST(stream), 
-      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)dgate_up, rows, F);
+  const bool vec = F % 8 == 0 && vec16(dy, gate_up, dgate_up);
+  launch_pdl(vec ? swiglu_bwd_kernel<true> : swiglu_bwd_kernel<false>, dim3(grid_for(rows * (vec ? F / 8 : F), 256)), dim3(256), 0, ST(stream),
+             (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)dgate_up, rows, F);
   return CHECK_LAUNCH();
 }
 extern "C" int incin_rope(void* x, long long B, int T, int H, int D, long long stride_b, long long stride_t,
                           long long stride_h, float theta, int inverse, void* stream) {
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0 || (D & 1)) return INCIN_ERR_ARGUMENT;
-  launch_pdl(rope_kernel, dim3(grid_for(B * T * H * (D / 2), 256)), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, B, T, H, D, stride_b,
-                                                                          stride_t, stride_h, theta, inverse);
+  const long long positions = B * T, blocks = (positions + ROPE_TOKENS - 1) / ROPE_TOKENS;
+  if (D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && vec16(x, x, x) && stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0 &&
+      blocks <= 0x7fffffffLL && (long long)H * D <= (1 << 24))
+    launch_pdl(rope_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, positions, T, H, D, stride_b, stride_t,
+               stride_h, theta, inverse);
+  else
+    launch_pdl(rope_kernel, dim3(grid_for(B * T * H * (D / 2), 256)), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, B, T, H, D, stride_b,
+               stride_t, stride_h, theta, inverse);
   return CHECK_LAUNCH();
 }
 extern "C" int incin_philox_uniform_f32(float* out, long long n, uint64_t seed, uint64_t offset, void* stream) {
