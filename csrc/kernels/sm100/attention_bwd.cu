@@ -61,6 +61,7 @@ struct FbParams {
   alignas(64) CUtensorMap tm_dq;   // fp32 dq_accum as {D, T, Hq, B}, 32 x 128 boxes (head_dim-64 kernel: bulk reduce-adds)
   int T, Hq, Hkv, n_tiles;
   int batch;           // B (the persistent kernel enumerates its work items itself)
+  int kv_major;        // head_dim 128: 1 = all heads' longest items first, 0 = a head's KV tiles are neighbours
   float scale, scale_log2;
   int Tpad;            // T rounded up to the tile edge: row stride of lse / delta
   const float* lse;    // [B, Hq, Tpad] log2 domain, +inf beyond T
@@ -639,11 +640,17 @@ static int launch_bwd(const incin_attn_desc* d, cudaStream_t stream) {
   p.dv_stride_h = d->dv_stride_h;
   p.status = (int*)d->status;
   p.prof = attn_prof_buffer();
+  p.kv_major = 0;
   dim3 grid(p.n_tiles, d->Hkv, d->B);
   if (use_split || use_steps) {   // persistent: one CTA per SM (or per item when there are fewer items)
     const long long items = (long long)p.n_tiles * d->Hkv * d->B;
     static const int sms = [] { int dev = 0, n = 148; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
     grid = dim3((unsigned)(items < sms ? items : sms), 1, 1);
+    // Few items per CTA: longest first over all heads, or one CTA draws two long ones (B 1, T 4096, H 24 / 8: 256 items,
+    // 703 -> 429 us; B 1, T 8191, H 24 / 8: 1708 -> 1268; B 4, T 4096, H 24 / 8: 1024 items, 1389 -> 1301; B 1, T 2048,
+    // H 32: 170 -> 153).  Many: a head's KV tiles stay neighbours, its fp32 dQ accumulator in L2 (B 8, T 4096, H 32: 8192
+    // items, 3626 us against 4651; B 8, T 700, H 32: 1536 items, 272 against 278).
+    p.kv_major = items <= 7 * sms;
   }
   if (launch_pdl<true>(kern, grid, dim3(FB_THREADS), smem_bytes, stream, tq, tk, tv, tdo, p) != cudaSuccess) return INCIN_ERR_LAUNCH;
   long long n8 = rows * D / 8;

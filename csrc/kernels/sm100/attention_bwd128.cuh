@@ -107,7 +107,7 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int heads_batches = p.Hkv * p.batch;
   const int n_items = p.n_tiles * heads_batches;
   const int n_steps_total = (p.T + TQ - 1) / TQ;     // 64-query steps of the whole sequence
-  // Item list: (batch, KV head) outermost, KV tile innermost, so the CTAs that run at the same time work on a handful
+  // Item list (unless kv_major, for launches of few items): (batch, KV head) outermost, KV tile innermost, so the CTAs that run at the same time work on a handful
   // of heads: their fp32 dQ accumulator (T x D x 4 bytes per head, touched by every KV tile of the head), Q and dO stay
   // in L2 between the KV tiles.  With the KV tile outermost 148 CTAs spread over 148 heads, the accumulator lines were
   // evicted between two adds and every add became a DRAM read-modify-write (twice the accumulator per KV tile).
@@ -117,8 +117,8 @@ flash_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int G = (int)gridDim.x, c = (int)blockIdx.x;
     const int idx = (r & 1) ? (r + 1) * G - 1 - c : r * G + c;
     if (idx >= n_items) return false;
-    kv_tile = idx % p.n_tiles;
-    const int hb = idx / p.n_tiles;
+    kv_tile = p.kv_major ? idx / heads_batches : idx % p.n_tiles;
+    const int hb = p.kv_major ? idx % heads_batches : idx / p.n_tiles;
     hkv = hb % p.Hkv;
     b = hb / p.Hkv;
     return true;

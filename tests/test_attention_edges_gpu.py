@@ -49,3 +49,30 @@ def test_forward_tile_edges(B, T, Hq, Hkv, D):
     # |error| <= 2^-8 (sum p |v| + |o|), 5 % above it for the fp32 scores, exponentials and sums
     bound = 2.0 ** -8 * 1.05 * (torch.einsum("bhqk,bkhd->bqhd", p, vd.abs()) + ref.abs()) + 1e-5
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 900, 6, 2), (9, 384, 40, 40), (2, 1500, 16, 8)])
+def test_backward_item_orders(B, T, Hq, Hkv):
+    """head_dim 128 walks its work items longest first over all heads (few items) or head by head (1080 items here)."""
+    from incin_b200.ops import attention as A
+    from incin_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(T)
+    q, k, v, do = (torch.randn(B, T, h, 128, generator=g).to(torch.bfloat16).cuda() for h in (Hq, Hkv, Hkv, Hq))
+    leaves = [t.requires_grad_() for t in (q, k, v)]
+    got = torch.autograd.grad(A.flash_attention(*leaves), leaves, do)
+    G.check_status()
+    grp, scale = Hq // Hkv, 128 ** -0.5
+    qf, kf, vf, df = (t.detach().double().transpose(1, 2) for t in (q, k.repeat_interleave(grp, 2), v.repeat_interleave(grp, 2), do))
+    mask = torch.ones(T, T, device="cuda", dtype=torch.bool).tril()
+    for b in range(B):
+        p = torch.softmax((qf[b] @ kf[b].mT * scale).masked_fill(~mask, float("-inf")), -1)
+        o, dp = p @ vf[b], df[b] @ vf[b].mT
+        delta = (df[b] * o).sum(-1, keepdim=True)
+        ds = p * (dp - delta)
+        # bf16 keeps 8 bits: P and dS are rounded before their products, O before delta = sum(dO O), the result at the end
+        e = p * ((dp - delta).abs() + (df[b] * o).abs().sum(-1, keepdim=True))
+        fold = lambda t: t.view(Hkv, grp, T, 128).sum(1)
+        refs = (scale * ds @ kf[b], fold(scale * ds.mT @ qf[b]), fold(p.mT @ df[b]))
+        slack = (scale * e @ kf[b].abs(), fold(scale * e.mT @ qf[b].abs()), fold(p.mT @ df[b].abs()))
+        for x, r, s in zip(got, refs, slack):
+            assert ((x[b].double().transpose(0, 1) - r).abs() <= 2.0 ** -8 * 1.05 * (s + r.abs()) + 1e-4).all()
