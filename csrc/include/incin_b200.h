@@ -179,6 +179,9 @@ int incin_swiglu_bwd(const void* dy, const void* gate_up, void* dgate_up, long l
 /* rotary embedding in place on [B][T][H][D] slices with row stride `ld`; inverse=1 applies the transpose (backward) */
 int incin_rope(void* x, long long B, int T, int H, int D, long long stride_b, long long stride_t, long long stride_h,
                float theta, int inverse, void* stream);
+/* The same from dense x [B, T, Htot, D] into dense y: heads [0, H) rotated, the others copied.  D % 16 == 0, D <= 256, both
+ * 16-byte aligned. */
+int incin_rope_out(const void* x, void* y, long long B, int T, int H, int Htot, int D, float theta, int inverse, void* stream);
 
 /* ---- optimiser --------------------------------------------------------------------------------- */
 /* hyper (device, 8 floats): {lr, beta1, beta2, eps, weight_decay, step, grad_scale, unused}.

@@ -270,10 +270,11 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long B, int T, i
 // The same for 16-byte aligned rows with D / 2 a multiple of 8 (at most ROPE_MAX_HALF).  A block takes ROPE_TOKENS
 // positions, works out their angles once for all heads (power, sine and cosine per pair and head were most of the general
 // kernel's time) and rotates eight pairs a thread with 16-byte accesses.  Bound by memory; 8192 positions, 36 heads of 64:
-// 57 -> 16 us.
+// 57 -> 16 us.  Reads x and writes y (the same buffer for the in-place call); heads H .. Ht - 1 are copied, so that the
+// caller who has to keep x does not copy it first (13 us there).
 constexpr int ROPE_TOKENS = 8, ROPE_MAX_HALF = 128;
-__global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict__ x, long long positions, int T, int H, int D, long long sb,
-                                                       long long st, long long sh, float theta, int inverse) {
+__global__ void __launch_bounds__(256) rope_vec_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, long long positions, int T, int H, int Ht,
+                                                       int D, long long sb, long long st, long long sh, float theta, int inverse) {
   pdl_launch_dependents();
   __shared__ float2 angle[ROPE_TOKENS * ROPE_MAX_HALF];
   const int half = D / 2, vecs = half / 8;
@@ -283,14 +284,19 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
     angle[i] = rope_angle((int)((first + i / half) % T), i % half, D, theta, inverse);
   __syncthreads();
   pdl_wait();
-  const int per = H * vecs;
+  const int per = Ht * vecs;
   for (int i = threadIdx.x; i < n * per; i += 256) {
     const int tok = i / per, k = i - tok * per, h = k / vecs, v = k - h * vecs;
     const long long pos = first + tok, b = pos / T;
-    __nv_bfloat16* p = x + b * sb + (pos - b * T) * st + (long long)h * sh + v * 8;
+    const long long off = b * sb + (pos - b * T) * st + (long long)h * sh + v * 8;
+    if (h >= H) {
+      *reinterpret_cast<uint4*>(y + off) = *reinterpret_cast<const uint4*>(x + off);
+      *reinterpret_cast<uint4*>(y + off + half) = *reinterpret_cast<const uint4*>(x + off + half);
+      continue;
+    }
     float a[8], c[8];
-    ld_bf16<true>(p, a);
-    ld_bf16<true>(p + half, c);
+    ld_bf16<true>(x + off, a);
+    ld_bf16<true>(x + off + half, c);
     const float2* cs = angle + tok * half + v * 8;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -299,8 +305,8 @@ __global__ void __launch_bounds__(256) rope_vec_kernel(__nv_bfloat16* __restrict
       c[e] = c[e] * q.x + a[e] * q.y;
       a[e] = r;
     }
-    st_bf16<true>(p, a);
-    st_bf16<true>(p + half, c);
+    st_bf16<true>(y + off, a);
+    st_bf16<true>(y + off + half, c);
   }
 }
 
@@ -445,14 +451,27 @@ extern "C" int incin_swiglu_bwd(const void* dy, const void* gate_up, void* dgate
              (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)dgate_up, rows, F);
   return CHECK_LAUNCH();
 }
+static bool rope_vec_ok(long long positions, int heads, int D) {
+  return D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && (positions + ROPE_TOKENS - 1) / ROPE_TOKENS <= 0x7fffffffLL &&
+         (long long)heads * D <= (1 << 24);
+}
+extern "C" int incin_rope_out(const void* x, void* y, long long B, int T, int H, int Htot, int D, float theta, int inverse, void* stream) {
+  if (!x || !y || B <= 0 || T <= 0 || H <= 0 || Htot < H || D <= 0 || (D & 1)) return INCIN_ERR_ARGUMENT;
+  const long long positions = B * T;
+  if (!rope_vec_ok(positions, Htot, D)) return INCIN_ERR_UNSUPPORTED;
+  if (!vec16(x, y, y)) return INCIN_ERR_ALIGNMENT;
+  launch_pdl(rope_vec_kernel, dim3((unsigned)((positions + ROPE_TOKENS - 1) / ROPE_TOKENS)), dim3(256), 0, ST(stream),
+             (const __nv_bfloat16*)x, (__nv_bfloat16*)y, positions, T, H, Htot, D, (long long)T * Htot * D, (long long)Htot * D, (long long)D,
+             theta, inverse);
+  return CHECK_LAUNCH();
+}
 extern "C" int incin_rope(void* x, long long B, int T, int H, int D, long long stride_b, long long stride_t,
                           long long stride_h, float theta, int inverse, void* stream) {
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0 || (D & 1)) return INCIN_ERR_ARGUMENT;
   const long long positions = B * T, blocks = (positions + ROPE_TOKENS - 1) / ROPE_TOKENS;
-  if (D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && vec16(x, x, x) && stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0 &&
-      blocks <= 0x7fffffffLL && (long long)H * D <= (1 << 24))
-    launch_pdl(rope_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, positions, T, H, D, stride_b, stride_t,
-               stride_h, theta, inverse);
+  if (rope_vec_ok(positions, H, D) && vec16(x, x, x) && stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0)
+    launch_pdl(rope_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream), (const __nv_bfloat16*)x, (__nv_bfloat16*)x, positions, T, H,
+               H, D, stride_b, stride_t, stride_h, theta, inverse);
   else
     launch_pdl(rope_kernel, dim3(grid_for(B * T * H * (D / 2), 256)), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, B, T, H, D, stride_b,
                stride_t, stride_h, theta, inverse);

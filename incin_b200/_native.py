@@ -98,6 +98,7 @@ _CUDA_SIGS = {
     "incin_swiglu_fwd": (c_int, [c_void_p, c_void_p, c_ll, c_int, c_void_p]),
     "incin_swiglu_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_void_p]),
     "incin_rope": (c_int, [c_void_p, c_ll, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_float, c_int, c_void_p]),
+    "incin_rope_out": (c_int, [c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p]),
     "incin_adamw_flat": (c_int, [c_void_p] * 5 + [c_ll, c_ll, c_void_p, c_void_p]),
     "incin_sgd_flat": (c_int, [c_void_p] * 4 + [c_ll, c_ll, c_void_p, c_void_p]),
     "incin_philox_uniform_f32": (c_int, [c_void_p, c_ll, c_u64, c_u64, c_void_p]),

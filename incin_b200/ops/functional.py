@@ -194,10 +194,11 @@ class _MLP(torch.autograd.Function):
     """y = act(x W1^T + b1) W2^T + b2 + residual; the activation backward rides in the dgrad GEMM epilogue."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, residual, act, defer_b2_grad=False):
+    def forward(ctx, x, w1, b1, w2, b2, residual, act, defer_b2_grad=False, keep_pre=True):
         x = _c(x)
         ctx.defer_b2 = defer_b2_grad
-        pre = torch.empty(*x.shape[:-1], w1.shape[0], dtype=torch.bfloat16, device=x.device)
+        # the pre-activation is only wanted by the backward
+        pre = torch.empty(*x.shape[:-1], w1.shape[0], dtype=torch.bfloat16, device=x.device) if keep_pre else None
         h = G.mm_nt(x, w1, bias=b1, act=act, aux=pre, max_ctas=_max_ctas)
         y = G.mm_nt(h, w2, bias=b2, residual=_c(residual) if residual is not None else None, max_ctas=_max_ctas)
         ctx.save_for_backward(x, w1, w2, pre, h)
@@ -224,13 +225,13 @@ class _MLP(torch.autograd.Function):
         _ready(w1)
         if ctx.b1 is not None:
             _ready(ctx.b1)
-        return dx, None, None, None, None, (dy if ctx.has_res else None), None, None
+        return dx, None, None, None, None, (dy if ctx.has_res else None), None, None, None
 
 
 def mlp(x, w1, b1, w2, b2, *, act="gelu", residual=None, defer_b2_grad: bool = False):
     """``defer_b2_grad``: the gradient of ``b2`` is produced by the norm that consumes the output (see :func:`linear`)."""
     if _nat(x):
-        return _MLP.apply(x, w1, b1, w2, b2, residual, ACT[act], defer_b2_grad and b2 is not None)
+        return _MLP.apply(x, w1, b1, w2, b2, residual, ACT[act], defer_b2_grad and b2 is not None, torch.is_grad_enabled())
     h = TF.linear(x, w1, b1)
     h = TF.gelu(h) if act == "gelu" else TF.silu(h)
     y = TF.linear(h, w2, b2)
@@ -549,19 +550,13 @@ class _Rope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, n_rot_heads, D, theta):
         # x: [B, T, Htot, D] packed heads; the first n_rot_heads heads (q and k) are rotated
-        x = _c(x).clone()
-        B, T, Ht, _ = x.shape
-        K.rope_(x, B, T, n_rot_heads, D, T * Ht * D, Ht * D, D, theta, False)
-        ctx.dims = (n_rot_heads, D, theta)
-        return x
+        ctx.dims = (n_rot_heads, theta)
+        return K.rope_out(_c(x), n_rot_heads, theta, False)
 
     @staticmethod
     def backward(ctx, dy):
-        n, D, theta = ctx.dims
-        dy = _c(dy).clone()
-        B, T, Ht, _ = dy.shape
-        K.rope_(dy, B, T, n, D, T * Ht * D, Ht * D, D, theta, True)
-        return dy, None, None, None
+        n, theta = ctx.dims
+        return K.rope_out(_c(dy), n, theta, True), None, None, None
 
 
 def _rope_cpu(x, n, D, theta):

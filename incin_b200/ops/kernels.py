@@ -217,6 +217,17 @@ def rope_(x, B, T, H, D, stride_b, stride_t, stride_h, theta, inverse, offset=0)
     return x
 
 
+def rope_out(x, n_rot, theta, inverse):
+    """Rotated copy of a dense ``[B, T, Htot, D]`` tensor: heads ``[0, n_rot)`` rotated, the others as they are."""
+    B, T, Ht, D = x.shape
+    if D % 16 or D > 256 or x.data_ptr() % 16 or x.numel() == 0:
+        y = x.clone()
+        return rope_(y, B, T, n_rot, D, T * Ht * D, Ht * D, D, theta, inverse)
+    y = torch.empty_like(x)
+    nat.check(nat.cuda().incin_rope_out(x.data_ptr(), y.data_ptr(), B, T, n_rot, Ht, D, theta, int(inverse), _s()), "rope_out")
+    return y
+
+
 def adamw_flat(master, m, v, grad, shadow, n_decay, hyper):
     nat.check(nat.cuda().incin_adamw_flat(master.data_ptr(), m.data_ptr(), v.data_ptr(), grad.data_ptr(),
                                          nat.ptr(shadow), master.numel(), n_decay, hyper.data_ptr(), _s()), "adamw")

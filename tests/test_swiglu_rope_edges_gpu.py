@@ -39,6 +39,9 @@ def test_rope(B, T, H, D, inverse):
     cs, sn = ang.cos().cuda()[None, :, None], ang.sin().cuda()[None, :, None] * (-1.0 if inverse else 1.0)
     a, c = ref[:, :, :H, :half].clone(), ref[:, :, :H, half:].clone()
     ref[:, :, :H, :half], ref[:, :, :H, half:] = a * cs - c * sn, c * cs + a * sn
+    y = K.rope_out(x, H, 10000.0, inverse)
+    assert torch.equal(y[:, :, H:], x[:, :, H:])
     K.rope_(x, B, T, H, D, T * (H + 2) * D, (H + 2) * D, D, 10000.0, inverse)
     # one rounding to bf16, and angles up to T in fp32 (2^-22 of the angle, hardware sine and cosine)
     assert ((x.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + (T * 2.0 ** -20 + 1e-5) * 4).all()
+    assert torch.equal(y, x)
