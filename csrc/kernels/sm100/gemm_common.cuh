@@ -176,7 +176,11 @@ __device__ __forceinline__ void epilogue_values(const GemmKernelParams& p, const
           }
           if (p.act == INCIN_ACT_GELU) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = gelu_erf(v[j]);
+            for (int j = 0; j < 32; j += 2) {
+              const float2 y = gelu_erf2(make_float2(v[j], v[j + 1]));
+              v[j] = y.x;
+              v[j + 1] = y.y;
+            }
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
@@ -193,8 +197,9 @@ __device__ __forceinline__ void epilogue_values(const GemmKernelParams& p, const
               for (int e = 0; e < 8; ++e) {
                 const float2 f = unpack_bf16x2(bw[e]);
                 if (p.act == INCIN_ACT_DGELU) {
-                  v[q * 16 + e * 2] *= gelu_erf_grad(f.x);
-                  v[q * 16 + e * 2 + 1] *= gelu_erf_grad(f.y);
+                  const float2 dg = gelu_erf_grad2(f);
+                  v[q * 16 + e * 2] *= dg.x;
+                  v[q * 16 + e * 2 + 1] *= dg.y;
                 } else {
                   v[q * 16 + e * 2] *= silu_grad(f.x);
                   v[q * 16 + e * 2 + 1] *= silu_grad(f.y);
@@ -210,8 +215,9 @@ __device__ __forceinline__ void epilogue_values(const GemmKernelParams& p, const
               for (int e = 0; e < 4; ++e) {
                 const float2 f = unpack_bf16x2(bw[e]);
                 if (p.act == INCIN_ACT_DGELU) {
-                  v[q * 8 + e * 2] *= gelu_erf_grad(f.x);
-                  v[q * 8 + e * 2 + 1] *= gelu_erf_grad(f.y);
+                  const float2 dg = gelu_erf_grad2(f);
+                  v[q * 8 + e * 2] *= dg.x;
+                  v[q * 8 + e * 2 + 1] *= dg.y;
                 } else {
                   v[q * 8 + e * 2] *= silu_grad(f.x);
                   v[q * 8 + e * 2 + 1] *= silu_grad(f.y);

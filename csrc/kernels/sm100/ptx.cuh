@@ -420,12 +420,67 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, bool a_mn_m
 // ---------------------------------------------------------------------------
 // small numeric helpers shared by kernels
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float gelu_erf(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_erf_grad(float x) {
-  const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
-  return cdf + x * pdf;
+// two fp32 operations in one issue slot (sm_100)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)), "l"(reinterpret_cast<uint64_t&>(c)));
+  return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;"
+      : "=l"(reinterpret_cast<uint64_t&>(d))
+      : "l"(reinterpret_cast<uint64_t&>(a)), "l"(reinterpret_cast<uint64_t&>(b)));
+  return d;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+// Normal distribution function Phi(x) and e = exp(-x^2 / 2), for the erf form of GELU.
+// Phi(-|x|) = e * f(|x|) with f(a) = erfcx(a / sqrt 2) / 2, smooth and bounded, is a degree-6 polynomial in
+// s = p a / (1 + p a) in [0, 1) with constant term 1/2 (the variable is the classical one of rational erfc
+// approximations; coefficients fitted here for the least maximum error of Phi, 5.2e-9).  In fp32 arithmetic, against
+// 64 bits on N(0, 2^2) and [-12, 12]: gelu rms 4.5e-8, max 3.8e-7, gradient rms 2.5e-8, max 1.3e-7; with an exactly
+// rounded erf in x / 2 (1 + erf) 5.1e-8, 4.5e-7, 2.6e-8, 1.35e-7, and its tail (x < -3) loses all digits but two where
+// this keeps four.  Two special-function operations and 14 packed ones instead of a call with a branch: the GEMM
+// epilogues with GELU were bound by it (8192 x 768 -> 3072: with GELU and side output 59 -> 51 us, data gradient
+// with GELU' 88 -> 71 us; 35 us without).  |x| is capped where e has long vanished, so that infinities
+// do not meet 0 in s; NaN arrives through e.
+__device__ __forceinline__ float2 normal_cdf2(float2 x, float2& e) {
+  const float2 u = mul2(mul2(x, x), both(-0.72134752f));   // -x^2 / (2 ln 2)
+  e = make_float2(exp2f(u.x), exp2f(u.y));
+  const float2 pa = mul2(make_float2(fminf(fabsf(x.x), 64.f), fminf(fabsf(x.y), 64.f)), both(0.275f));
+  const float2 d = add2(pa, both(1.f));
+  const float2 s = mul2(pa, make_float2(__fdividef(1.f, d.x), __fdividef(1.f, d.y)));
+  float2 r = both(-0x1.e52a92p-4f);
+  r = fma2(r, s, both(0x1.ed9d88p-3f));
+  r = fma2(r, s, both(0x1.a2f704p-3f));
+  r = fma2(r, s, both(-0x1.3b84acp+0f));
+  r = fma2(r, s, both(0x1.dae3a4p+0f));
+  r = fma2(r, s, both(-0x1.7360f6p+0f));
+  r = fma2(r, s, both(0.5f));
+  const float2 q = mul2(r, e), c = fma2(mul2(r, both(-1.f)), e, both(1.f));
+  return make_float2(x.x >= 0.f ? c.x : q.x, x.y >= 0.f ? c.y : q.y);
+}
+__device__ __forceinline__ float2 gelu_erf2(float2 x) {
+  float2 e;
+  return mul2(x, normal_cdf2(x, e));
+}
+__device__ __forceinline__ float2 gelu_erf_grad2(float2 x) {
+  float2 e;
+  const float2 c = normal_cdf2(x, e);
+  return fma2(mul2(x, both(0.3989422804014327f)), e, c);
+}
+__device__ __forceinline__ float gelu_erf(float x) { return gelu_erf2(make_float2(x, x)).x; }
+__device__ __forceinline__ float gelu_erf_grad(float x) { return gelu_erf_grad2(make_float2(x, x)).x; }
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
 __device__ __forceinline__ float silu_grad(float x) {
   const float s = 1.0f / (1.0f + __expf(-x));
