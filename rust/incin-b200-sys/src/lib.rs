@@ -175,6 +175,7 @@ extern "C" {
     pub fn incin_coll_all_to_all(bufs: *const *mut c_void, world: c_int, rank: c_int, offset_bytes: c_longlong, chunk_bytes: c_longlong, out: *mut c_void, stream: *mut c_void) -> c_int;
     pub fn incin_coll_reduce(bufs: *const *mut c_void, world: c_int, offset_bytes: c_longlong, first_elem: c_longlong, n: c_longlong, op: c_int, is_bf16: c_int, out: *mut c_void, stream: *mut c_void) -> c_int;
     pub fn incin_colsum_accum(dy: *const c_void, dbias: *mut f32, rows: c_longlong, N: c_int, ld: c_longlong, stream: *mut c_void) -> c_int;
+    pub fn incin_colsum_accum_typed(dy: *const c_void, dbias: *mut f32, rows: c_longlong, N: c_int, ld: c_longlong, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_conv_out_hw(g: *const incin_conv_geom, oh: *mut c_int, ow: *mut c_int) -> c_int;
     pub fn incin_cpu_adamw_f32(w: *mut f32, m: *mut f32, v: *mut f32, g: *const f32, n: i64, lr: f32, b1: f32, b2: f32, eps: f32, wd: f32, step: c_int);
     pub fn incin_cpu_attention_f32(q: *const f32, k: *const f32, v: *const f32, o: *mut f32, heads: i64, T: i64, D: i64, scale: f32, causal: c_int);
@@ -257,6 +258,7 @@ extern "C" {
     pub fn incin_rmsnorm_bwd(dy: *const c_void, x: *const c_void, gamma: *const c_void, rstd: *const f32, dx_add: *const c_void, dx: *mut c_void, dgamma: *mut f32, scratch: *mut f32, rows: c_longlong, C: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_rmsnorm_fwd(x: *const c_void, gamma: *const c_void, y: *mut c_void, rstd: *mut f32, rows: c_longlong, C: c_int, eps: f32, stream: *mut c_void) -> c_int;
     pub fn incin_rope(x: *mut c_void, B: c_longlong, T: c_int, H: c_int, D: c_int, stride_b: c_longlong, stride_t: c_longlong, stride_h: c_longlong, theta: f32, inverse: c_int, stream: *mut c_void) -> c_int;
+    pub fn incin_rope_out(x: *const c_void, y: *mut c_void, B: c_longlong, T: c_int, H: c_int, Htot: c_int, D: c_int, theta: f32, inverse: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_scatter_add_rows(src: *const c_void, index: *const c_longlong, dst: *mut f32, n_idx: c_longlong, row_elems: c_longlong, dst_rows: c_longlong, src_is_bf16: c_int, err_flag: *mut c_int, stream: *mut c_void) -> c_int;
     pub fn incin_scatter_last(src: *const c_void, index: *const c_longlong, dst: *mut c_void, rows: c_longlong, n_dst: c_longlong, n_idx: c_longlong, elem_bytes: c_int, err_flag: *mut c_int, stream: *mut c_void) -> c_int;
     pub fn incin_sgd_flat(master: *mut f32, mom: *mut f32, grad: *const f32, shadow_bf16: *mut c_void, n: c_longlong, n_decay: c_longlong, hyper: *const f32, stream: *mut c_void) -> c_int;
@@ -291,6 +293,7 @@ extern "C" {
     pub fn incin_telemetry_open(path: *const c_char, capacity: i64) -> i64;
     pub fn incin_telemetry_raw(h: i64, json_line: *const c_char) -> c_int;
     pub fn incin_telemetry_scalar(h: i64, name: *const c_char, value: f64, step: i64) -> c_int;
+    pub fn incin_transpose_f32(src: *const f32, dst: *mut f32, rows: c_longlong, cols: c_longlong, colsum: *mut f32, stream: *mut c_void) -> c_int;
     pub fn incin_tri(x: *const c_void, out: *mut c_void, batch: c_longlong, rows: c_longlong, cols: c_longlong, diagonal: c_longlong, upper: c_int, elem_bytes: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_where(cond: *const u8, a: *const c_void, b: *const c_void, out: *mut c_void, n: c_longlong, elem_bytes: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_xent_bwd(logits: *mut c_void, targets: *const i64, lse: *const f32, dloss: *const f32, scale: f32, rows: c_longlong, V: c_int, ld: c_longlong, stream: *mut c_void) -> c_int;
