@@ -465,7 +465,8 @@ norm_bwd_param_final(const float* __restrict__ scratch, float* __restrict__ dgam
 // 1024 < C <= 4096 (C % 8 == 0): a block holds a row, eight columns a thread, so gamma and the column's partial sums stay
 // in registers while the block walks its rows; the next row is requested before the block meets to add up the current
 // one.  Bound by memory: x, dy and dx_add read once, dx written.  The row-per-warp kernel read x and dy twice for dx and
-// the partial-sum kernel a third time.  8192 x 2048 RMS with dx_add: 54 -> 32 us with the final reduction.
+// the partial-sum kernel a third time.  8192 x 2048 RMS with dx_add: 54 -> 32 us with the final reduction
+// inside a training step, 66 -> 42 us with a cold L2; LayerNorm 65536 x 4096: 720 -> 509 us.
 // Block b takes rows b, b + gridDim.x, ... and writes scratch[b][{g}] (RMS) or scratch[b][{g, b}]; fixed order.
 __device__ __forceinline__ uint4 ld_row16(const __nv_bfloat16* p) {   // volatile: stays where the pipeline wants it
   uint4 v;
