@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict
   __shared__ T tile[64 * PITCH];
   const T* s = src + blockIdx.z * s_batch;
   T* d = dst + blockIdx.z * d_batch;
-  const long long c0 = (long long)blockIdx.x * 64, r0 = (long long)blockIdx.y * 64;
+  const unsigned tiles_c = (unsigned)((cols + 63) / 64);   // column tiles fastest, in one grid axis: no limit on either side
+  const long long c0 = (long long)(blockIdx.x % tiles_c) * 64, r0 = (long long)(blockIdx.x / tiles_c) * 64;
   const int tv = (threadIdx.x % TPR) * V, tr = threadIdx.x / TPR;
   float sum[V];
   if constexpr (COLSUM) {
@@ -218,11 +219,12 @@ inline unsigned grid_for(long long n, int block) {
   return (unsigned)(g < 1 ? 1 : (g > 148LL * 16 ? 148LL * 16 : g));
 }
 
-// src [batch, rows, cols] -> dst [batch, cols, rows], both dense; at most 65535 batches and 65535 x 64 rows
+// src [batch, rows, cols] -> dst [batch, cols, rows], both dense; at most 65535 batches and 2^31 - 1 tiles each
+inline long long transpose_tiles(long long rows, long long cols) { return ((rows + 63) / 64) * ((cols + 63) / 64); }
 template <typename T, bool COLSUM>
 int transpose_launch(const T* src, T* dst, long long rows, long long cols, long long batch, float* colsum, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
-  const dim3 grid((unsigned)((cols + 63) / 64), (unsigned)((rows + 63) / 64), (unsigned)batch);
+  const dim3 grid((unsigned)transpose_tiles(rows, cols), 1, (unsigned)batch);
   const bool vec = rows % V == 0 && cols % V == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
   if (vec) transpose_tile_kernel<T, true, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
   else transpose_tile_kernel<T, false, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
@@ -241,7 +243,7 @@ int strided_copy_t(const void* src, void* dst, const Geometry& g, cudaStream_t s
       g.sstride[last - 1] == 1 && g.sstride[last] == g.shape[last - 1]) {
     const long long rows = g.shape[last], cols = g.shape[last - 1];   // source is [.., rows(last), cols(last-1)] dense
     const long long batch = g.rank == 3 ? g.shape[0] : 1;
-    if (batch <= 65535 && (rows + 63) / 64 <= 65535 && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols))) {
+    if (batch <= 65535 && transpose_tiles(rows, cols) <= 0x7fffffffLL && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols))) {
       return transpose_launch<T, false>(static_cast<const T*>(src), static_cast<T*>(dst), rows, cols, batch, nullptr, s);
     }
   }
@@ -305,7 +307,7 @@ extern "C" int incin_strided_copy(const void* src, void* dst, int rank, const lo
 
 extern "C" int incin_transpose_f32(const float* src, float* dst, long long rows, long long cols, float* colsum, void* stream) {
   if (!src || !dst || rows <= 0 || cols <= 0) return INCIN_ERR_ARGUMENT;
-  if ((rows + 63) / 64 > 65535) return INCIN_ERR_TOO_LARGE;
+  if (transpose_tiles(rows, cols) > 0x7fffffffLL) return INCIN_ERR_TOO_LARGE;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   return colsum ? transpose_launch<float, true>(src, dst, rows, cols, 1, colsum, s)
                 : transpose_launch<float, false>(src, dst, rows, cols, 1, nullptr, s);

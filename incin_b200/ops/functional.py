@@ -107,8 +107,9 @@ class _LinearF32Acc(torch.autograd.Function):
     through autograd.  The tensor cores read 16-bit operands of the backward products as they lie; tf32 operands have to
     run along the reduction, so those are transposed first, the output gradient together with its column sums.
 
-    fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 290 -> 208 us and
-    273 -> 231 us a pass against products in fp32 with separate bias, conversion and transposition passes."""
+    fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 288 -> 168 us and
+    271 -> 183 us a pass against products in fp32 with separate bias, conversion and transposition passes (both bound by
+    the host now; 80 us on the device for fp16)."""
 
     @staticmethod
     def forward(ctx, x, w, b):
