@@ -114,11 +114,14 @@ class _LinearF32Acc(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b):
         x2 = _c(x).reshape(-1, x.shape[-1])
-        fused = b is None or (b.dtype == x.dtype and b.is_contiguous() and b.is_cuda)
+        # the epilogue reads one bias element per output column; any other bias is broadcast, or refused, by torch
+        fused = b is None or (b.shape == w.shape[:1] and b.dtype == x.dtype and b.is_contiguous() and b.is_cuda)
         if fused:
             y = G.mm_linear_other(x2, _c(w), b)
         else:
-            y = (G.mm_nt_f32out(x2, _c(w)) + b.float()).to(x.dtype)
+            y = G.mm_nt_f32out(x2, _c(w))
+            y += b.float()
+            y = y.to(x.dtype)
         ctx.save_for_backward(x2, w)
         ctx.has_bias = b is not None
         ctx.shape = x.shape

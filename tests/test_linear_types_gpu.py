@@ -31,6 +31,33 @@ def test_linear_forward_backward(dtype, rows, n_in, n_out):
     assert ((db.double() - dyd.sum(0)).abs() <= bound + 1e-6).all() and db.dtype == dtype
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1,), (), (40,), (1, 40), (9, 1), (9, 40)])
+def test_linear_bias_broadcast(dtype, shape):
+    """A bias that is not one element per output column is broadcast over the result as torch does it."""
+    from incin_b200.core.policy import MathMode, policy_scope
+    from incin_b200.ops import functional as F
+    g = torch.Generator().manual_seed(len(shape))
+    x, w, b = (torch.randn(s, generator=g).to(dtype).cuda() for s in ((9, 24), (40, 24), shape))
+    with policy_scope(math=MathMode.FAST):
+        y = F.linear(x, w, b)
+    ref = x.double() @ w.double().t() + b.double()
+    # as test_linear_forward_backward: one rounding for fp16, factors cut to 11 bits for fp32
+    u = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -9
+    bound = u * ref.abs() + (2.0 ** -20 if dtype == torch.float16 else u) * (x.double().abs() @ w.double().abs().t()) + 1e-6
+    assert y.dtype == dtype and ((y.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(39,), (41,), (0,), (1, 1, 40), (8, 40)])
+def test_linear_bias_refused(dtype, shape):
+    from incin_b200.core.policy import MathMode, policy_scope
+    from incin_b200.ops import functional as F
+    with policy_scope(math=MathMode.FAST), pytest.raises(RuntimeError):
+        F.linear(torch.zeros(9, 24, dtype=dtype, device="cuda"), torch.zeros(40, 24, dtype=dtype, device="cuda"),
+                 torch.zeros(shape, dtype=dtype, device="cuda"))
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
 @pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48), (1, 4194400, 1), (1, 1, 4194500)])
 def test_transpose_tiles(dtype, batch, rows, cols):
