@@ -165,6 +165,10 @@ int incin_causal_softmax_bwd(void* dp, const void* p, long long batch, int T, fl
 int incin_colsum_accum(const void* dy, float* dbias, long long rows, int N, long long ld, void* stream);
 /* the same with dy of type INCIN_GEMM_IN_BF16, _FP16 or _TF32 (= fp32); the sums are fp32 */
 int incin_colsum_accum_typed(const void* dy, float* dbias, long long rows, int N, long long ld, int dtype, void* stream);
+/* out[n] = sum_m dy[m][n] in dy's type, added up in fp32 in a fixed order (repeats to the bit); scratch: fp32,
+ * incin_colsum_scratch_floats(rows, N) elements */
+long long incin_colsum_scratch_floats(long long rows, int N);
+int incin_colsum_typed(const void* dy, void* out, float* scratch, long long rows, int N, long long ld, int dtype, void* stream);
 /* out[0] += sum(x^2); out[1] = 1.0 if any element is NaN/Inf (device-side gradient check, no D2H of tensors) */
 int incin_sumsq_nonfinite_f32(const float* x, long long n, float* out, void* stream);
 int incin_fill_f32(float* x, float value, long long n, void* stream);

@@ -292,8 +292,9 @@ __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__half v) { return __half2float(v); }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// block = 32 x 8 threads covering 64 columns; grid.y row chunks; fp32 atomics into the gradient buffer
-template <typename T>
+// block = 32 x 8 threads covering 64 columns; grid.y row chunks; fp32 atomics into the gradient buffer, or with PART the
+// chunk's sums into row blockIdx.y of a [chunks][N] buffer
+template <typename T, bool PART>
 __global__ void __launch_bounds__(256)
 colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long rows, int N, long long ld, int chunks) {
   pdl_launch_dependents();
@@ -329,7 +330,8 @@ colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long row
         float t = 0.f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) t += sh[k][tx * 2 + e];
-        atomicAdd(dbias + c0 + e, t);
+        if constexpr (PART) dbias[(long long)blockIdx.y * N + c0 + e] = t;
+        else atomicAdd(dbias + c0 + e, t);
       }
     }
   }
@@ -337,7 +339,7 @@ colsum_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long row
 
 // 16-byte variant: 32 lanes x VEC columns (8 of 16 bits, 4 fp32) per block, 8 row lanes; needs N % VEC == 0 and
 // ld % VEC == 0
-template <typename T>
+template <typename T, bool PART>
 __global__ void __launch_bounds__(256)
 colsum_vec_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long rows, int N, long long ld, int chunks) {
   pdl_launch_dependents();
@@ -368,25 +370,56 @@ colsum_vec_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
-    atomicAdd(dbias + c, t);
+    if constexpr (PART) dbias[(long long)blockIdx.y * N + c] = t;
+    else atomicAdd(dbias + c, t);
   }
 }
 
+// Second stage of the column sum with a fixed order: a block adds the partial sums of 32 columns, 32 lanes a column.
 template <typename T>
-static int colsum_launch(const void* dy, float* dbias, long long rows, int N, long long ld, cudaStream_t stream) {
+__global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restrict__ part, T* __restrict__ out, int N, int chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float sh[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  float a = 0.f;
+  if (c < N)
+    for (int k = ty; k < chunks; k += 32) a += part[(long long)k * N + c];
+  sh[ty][tx] = a;
+  __syncthreads();
+  a = warp_sum_f(sh[tx][ty]);
+  if (tx == 0 && blockIdx.x * 32 + ty < N) out[blockIdx.x * 32 + ty] = T(a);
+}
+
+// 16-byte form: enough chunks for four blocks on every SM, of 32 rows or more; else chunks of 256 rows, 128 at most
+static long long colsum_vec_chunks(long long rows, int colblocks) {
+  const long long want = (148 * 4 + colblocks - 1) / colblocks, most = (rows + 31) / 32;
+  return want < most ? want : most;
+}
+static long long colsum_plain_chunks(long long rows) {
+  const long long c = (rows + 255) / 256;
+  return c < 128 ? c : 128;
+}
+
+// dbias: the gradient buffer to add to, or (PART) the buffer of partial sums; *n_chunks: how many rows of it were written
+template <typename T, bool PART>
+static int colsum_launch(const void* dy, float* dbias, long long rows, int N, long long ld, cudaStream_t stream, int* n_chunks = nullptr) {
   constexpr int VEC = 16 / sizeof(T);
-  cudaError_t e;
-  if ((N % VEC) == 0 && (ld % VEC) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0) {
-    const int colblocks = (N + 32 * VEC - 1) / (32 * VEC);
-    long long chunks = (148 * 4 + colblocks - 1) / colblocks;
-    if (chunks > (rows + 31) / 32) chunks = (rows + 31) / 32;
-    if (chunks < 1) chunks = 1;
-    e = launch_pdl(colsum_vec_kernel<T>, dim3(colblocks, (unsigned)chunks), dim3(256), 0, stream, (const T*)dy, dbias, rows, N, ld, (int)chunks);
-  } else {
-    long long chunks = (rows + 255) / 256;
-    if (chunks > 128) chunks = 128;
-    e = launch_pdl(colsum_kernel<T>, dim3((N + 63) / 64, (unsigned)chunks), dim3(256), 0, stream, (const T*)dy, dbias, rows, N, ld, (int)chunks);
-  }
+  const bool vec = (N % VEC) == 0 && (ld % VEC) == 0 && (reinterpret_cast<uintptr_t>(dy) & 15) == 0;
+  const int colblocks = vec ? (N + 32 * VEC - 1) / (32 * VEC) : (N + 63) / 64;
+  const int chunks = (int)(vec ? colsum_vec_chunks(rows, colblocks) : colsum_plain_chunks(rows));
+  if (n_chunks) *n_chunks = chunks;
+  const cudaError_t e = launch_pdl(vec ? colsum_vec_kernel<T, PART> : colsum_kernel<T, PART>, dim3(colblocks, (unsigned)chunks), dim3(256), 0,
+                                   stream, (const T*)dy, dbias, rows, N, ld, chunks);
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
+}
+
+template <typename T>
+static int colsum_out(const void* dy, void* out, float* scratch, long long rows, int N, long long ld, cudaStream_t stream) {
+  int chunks = 0;
+  const int rc = colsum_launch<T, true>(dy, scratch, rows, N, ld, stream, &chunks);
+  if (rc != INCIN_OK) return rc;
+  const cudaError_t e = launch_pdl(colsum_final_kernel<T>, dim3((N + 31) / 32), dim3(1024), 0, stream, (const float*)scratch, (T*)out, N, chunks);
   return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
@@ -467,8 +500,25 @@ extern "C" int incin_colsum_accum(const void* dy, float* dbias, long long rows, 
 extern "C" int incin_colsum_accum_typed(const void* dy, float* dbias, long long rows, int N, long long ld, int dtype, void* stream) {
   if (rows <= 0 || N <= 0) return INCIN_ERR_ARGUMENT;
   const cudaStream_t s = (cudaStream_t)stream;
-  if (dtype == INCIN_GEMM_IN_BF16) return colsum_launch<__nv_bfloat16>(dy, dbias, rows, N, ld, s);
-  if (dtype == INCIN_GEMM_IN_FP16) return colsum_launch<__half>(dy, dbias, rows, N, ld, s);
-  if (dtype == INCIN_GEMM_IN_TF32) return colsum_launch<float>(dy, dbias, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_BF16) return colsum_launch<__nv_bfloat16, false>(dy, dbias, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_FP16) return colsum_launch<__half, false>(dy, dbias, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_TF32) return colsum_launch<float, false>(dy, dbias, rows, N, ld, s);
+  return INCIN_ERR_ARGUMENT;
+}
+
+extern "C" long long incin_colsum_scratch_floats(long long rows, int N) {
+  if (rows <= 0 || N <= 0) return 0;
+  const long long vec = colsum_vec_chunks(rows, (N + 255) / 256), plain = colsum_plain_chunks(rows);
+  return (vec > plain ? vec : plain) * N;
+}
+
+// Two stages in a fixed order, so that the sums repeat to the bit (the bias gradients that are returned as tensors; the
+// ones that accumulate into a flat buffer use atomics)
+extern "C" int incin_colsum_typed(const void* dy, void* out, float* scratch, long long rows, int N, long long ld, int dtype, void* stream) {
+  if (!dy || !out || !scratch || rows <= 0 || N <= 0) return INCIN_ERR_ARGUMENT;
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == INCIN_GEMM_IN_BF16) return colsum_out<__nv_bfloat16>(dy, out, scratch, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_FP16) return colsum_out<__half>(dy, out, scratch, rows, N, ld, s);
+  if (dtype == INCIN_GEMM_IN_TF32) return colsum_out<float>(dy, out, scratch, rows, N, ld, s);
   return INCIN_ERR_ARGUMENT;
 }

@@ -24,6 +24,7 @@ import torch
 import torch.nn.functional as TF
 
 from .. import _native as nat
+from ..core.policy import Determinism, MathMode, current_policy
 from . import gemm as G
 from . import kernels as K
 
@@ -105,7 +106,8 @@ class _LinearF32Acc(torch.autograd.Function):
     """Linear for fp16 tensors and, under ``MathMode.FAST``, fp32 tensors (multiplied as tf32) on the same tcgen05
     kernel as the bf16 path: fp32 accumulation, bias in the epilogue, rounded once to the input type.  Gradients return
     through autograd.  The tensor cores read 16-bit operands of the backward products as they lie; tf32 operands have to
-    run along the reduction, so those are transposed first, the output gradient together with its column sums.
+    run along the reduction, so those are transposed first.  Sums have a fixed order, but for the fp32 weight gradient,
+    whose order is only fixed under ``Determinism.REQUIRED``.
 
     fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 288 -> 168 us and
     271 -> 183 us a pass against products in fp32 with separate bias, conversion and transposition passes (both bound by
@@ -124,6 +126,8 @@ class _LinearF32Acc(torch.autograd.Function):
             y = y.to(x.dtype)
         ctx.save_for_backward(x2, w)
         ctx.has_bias = b is not None
+        # the policy belongs to the calling thread, and autograd runs the backward on one of its own
+        ctx.fixed_order = current_policy().determinism is Determinism.REQUIRED
         ctx.shape = x.shape
         return y.reshape(*x.shape[:-1], w.shape[0])
 
@@ -136,9 +140,6 @@ class _LinearF32Acc(torch.autograd.Function):
         half = dy2.dtype == torch.float16
         unit = 8 if half else 4
         dx = dw = db = None
-        db32 = None
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db32 = torch.zeros(n_out, dtype=torch.float32, device=dy.device)
         if ctx.needs_input_grad[0]:
             if n_out % unit:
                 dx = dy2 @ w
@@ -156,15 +157,14 @@ class _LinearF32Acc(torch.autograd.Function):
                 dw = dy2.t() @ x2
             elif half:
                 dw = G.mm_linear_other(dy2.t().contiguous(), x2.t().contiguous())
+            elif ctx.fixed_order:
+                dw = G.mm_linear_other(K.transpose_f32(dy2), K.transpose_f32(x2))
             else:
                 # the reduction over the rows is split among CTAs that add up in fp32
                 dw = torch.zeros(n_out, n_in, dtype=torch.float32, device=dy.device)
-                G.mm_nt_f32out(K.transpose_f32(dy2, db32), K.transpose_f32(x2), out=dw, accumulate=True, splits=0)
-                if db32 is not None:
-                    db, db32 = db32, None
-        if db32 is not None:
-            K.colsum_accum(dy2, db32)
-            db = db32.to(dy.dtype)
+                G.mm_nt_f32out(K.transpose_f32(dy2), K.transpose_f32(x2), out=dw, accumulate=True, splits=0)
+        if ctx.has_bias and ctx.needs_input_grad[2]:
+            db = K.colsum(dy2)
         return dx, dw, db
 
 
@@ -175,7 +175,6 @@ def _f32acc_native(x: torch.Tensor, w: torch.Tensor) -> bool:
     if x.dtype == torch.float16:
         return x.shape[-1] % 8 == 0
     if x.dtype == torch.float32:
-        from ..core.policy import MathMode, current_policy
         return current_policy().math == MathMode.FAST and x.shape[-1] % 4 == 0
     return False
 
@@ -356,7 +355,6 @@ class _Embedding(torch.autograd.Function):
     def backward(ctx, dout):
         (tokens,) = ctx.saved_tensors
         wte, wpe = ctx.wte, ctx.wpe
-        from ..core.policy import Determinism, current_policy
         if current_policy().determinism is Determinism.REQUIRED and not torch.cuda.is_current_stream_capturing():
             # fixed summation order: sort by token, one block per distinct token (not capturable: the number of
             # distinct tokens is read back to size the launch)

@@ -154,6 +154,18 @@ def colsum_accum(dy, dbias):
               "colsum")
 
 
+def colsum(dy):
+    """Column sums of ``dy [..., N]`` in its own type: fp32 inside, one rounding, the same bits every time."""
+    N = dy.shape[-1]
+    rows = dy.numel() // N
+    lib = nat.cuda()
+    out = torch.empty(N, dtype=dy.dtype, device=dy.device)
+    part = torch.empty(lib.incin_colsum_scratch_floats(rows, N), dtype=F32, device=dy.device)
+    nat.check(lib.incin_colsum_typed(dy.data_ptr(), out.data_ptr(), part.data_ptr(), rows, N, N, _COLSUM_KIND[dy.dtype], _s()),
+              "colsum")
+    return out
+
+
 def transpose_f32(x, colsum=None):
     """Dense transpose of a dense fp32 matrix; ``colsum`` (fp32), if given, gets the column sums of ``x`` added."""
     rows, cols = x.shape

@@ -58,6 +58,29 @@ def test_linear_bias_refused(dtype, shape):
                  torch.zeros(shape, dtype=dtype, device="cuda"))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,n_in,n_out", [(8184, 256, 200), (4096, 64, 72), (515, 64, 36), (3001, 64, 33)])
+def test_linear_gradients_repeat(dtype, rows, n_in, n_out):
+    """Under ``Determinism.REQUIRED`` (asked for around the forward; the backward runs on a thread of autograd) every
+    gradient repeats to the bit; bias gradients do without it."""
+    from incin_b200.core.policy import Determinism, MathMode, policy_scope
+    from incin_b200.ops import functional as F
+    g = torch.Generator().manual_seed(rows)
+    x, w, b, dy = (torch.randn(*s, generator=g).to(dtype).cuda() for s in ((rows, n_in), (n_out, n_in), (n_out,), (rows, n_out)))
+    x, w, b = (t.requires_grad_() for t in (x, w, b))
+    def grads(determinism):
+        with policy_scope(math=MathMode.FAST, determinism=determinism):
+            y = F.linear(x, w, b)
+        return torch.autograd.grad(y, (x, w, b), dy)
+    first = grads(Determinism.REQUIRED)
+    for _ in range(12):
+        assert all(torch.equal(p, q) for p, q in zip(grads(Determinism.REQUIRED), first))
+        assert torch.equal(grads(Determinism.PERMITTED)[2], first[2])
+    # at most 64 additions on the way of a term into its sum, each within 2^-24 of the magnitudes; one rounding to fp16
+    ref = dy.double().sum(0)
+    assert ((first[2].double() - ref).abs() <= 2.0 ** -11 * ref.abs() * (dtype == torch.float16) + 2.0 ** -18 * dy.double().abs().sum(0)).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
 @pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48), (1, 4194400, 1), (1, 1, 4194500)])
 def test_transpose_tiles(dtype, batch, rows, cols):
