@@ -169,6 +169,8 @@ int incin_colsum_accum_typed(const void* dy, float* dbias, long long rows, int N
  * incin_colsum_scratch_floats(rows, N) elements */
 long long incin_colsum_scratch_floats(long long rows, int N);
 int incin_colsum_typed(const void* dy, void* out, float* scratch, long long rows, int N, long long ld, int dtype, void* stream);
+/* out[n] = sum_k part[k][n], k < chunks, in a fixed order; out of type dtype */
+int incin_colsum_reduce(const float* part, void* out, long long chunks, int N, int dtype, void* stream);
 /* out[0] += sum(x^2); out[1] = 1.0 if any element is NaN/Inf (device-side gradient check, no D2H of tensors) */
 int incin_sumsq_nonfinite_f32(const float* x, long long n, float* out, void* stream);
 int incin_fill_f32(float* x, float value, long long n, void* stream);
@@ -258,7 +260,8 @@ int incin_cumsum(const void* x, void* out, long long outer, long long n, long lo
  * (0 = broadcast): transpose, narrow, paste, broadcast, concat and pad are all this one copy. */
 int incin_strided_copy(const void* src, void* dst, int rank, const long long* shape, const long long* src_strides,
                        const long long* dst_strides, int elem_bytes, void* stream);
-/* dst[cols][rows] = src[rows][cols] (both dense); colsum, if not NULL: colsum[c] += sum_r src[r][c] */
+/* dst[cols][rows] = src[rows][cols] (both dense); colsum, if not NULL, fp32 [ceil(rows / 64)][cols]: the column sums of each
+ * band of 64 rows, for incin_colsum_reduce */
 int incin_transpose_f32(const float* src, float* dst, long long rows, long long cols, float* colsum, void* stream);
 /* Indexed ops check every index: an out-of-range one is skipped and *err_flag (device int, may be NULL) is set. */
 int incin_gather_rows(const void* src, const long long* index, void* out, long long n_idx, long long row_elems,

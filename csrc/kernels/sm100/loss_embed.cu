@@ -377,14 +377,14 @@ colsum_vec_kernel(const T* __restrict__ dy, float* __restrict__ dbias, long long
 
 // Second stage of the column sum with a fixed order: a block adds the partial sums of 32 columns, 32 lanes a column.
 template <typename T>
-__global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restrict__ part, T* __restrict__ out, int N, int chunks) {
+__global__ void __launch_bounds__(1024) colsum_final_kernel(const float* __restrict__ part, T* __restrict__ out, int N, long long chunks) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float sh[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
   float a = 0.f;
   if (c < N)
-    for (int k = ty; k < chunks; k += 32) a += part[(long long)k * N + c];
+    for (long long k = ty; k < chunks; k += 32) a += part[k * N + c];
   sh[ty][tx] = a;
   __syncthreads();
   a = warp_sum_f(sh[tx][ty]);
@@ -415,12 +415,16 @@ static int colsum_launch(const void* dy, float* dbias, long long rows, int N, lo
 }
 
 template <typename T>
+static int colsum_final(const float* part, void* out, int N, long long chunks, cudaStream_t stream) {
+  const cudaError_t e = launch_pdl(colsum_final_kernel<T>, dim3((N + 31) / 32), dim3(1024), 0, stream, part, (T*)out, N, chunks);
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
+}
+
+template <typename T>
 static int colsum_out(const void* dy, void* out, float* scratch, long long rows, int N, long long ld, cudaStream_t stream) {
   int chunks = 0;
   const int rc = colsum_launch<T, true>(dy, scratch, rows, N, ld, stream, &chunks);
-  if (rc != INCIN_OK) return rc;
-  const cudaError_t e = launch_pdl(colsum_final_kernel<T>, dim3((N + 31) / 32), dim3(1024), 0, stream, (const float*)scratch, (T*)out, N, chunks);
-  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
+  return rc == INCIN_OK ? colsum_final<T>(scratch, out, N, chunks, stream) : rc;
 }
 
 }  // namespace incin
@@ -520,5 +524,14 @@ extern "C" int incin_colsum_typed(const void* dy, void* out, float* scratch, lon
   if (dtype == INCIN_GEMM_IN_BF16) return colsum_out<__nv_bfloat16>(dy, out, scratch, rows, N, ld, s);
   if (dtype == INCIN_GEMM_IN_FP16) return colsum_out<__half>(dy, out, scratch, rows, N, ld, s);
   if (dtype == INCIN_GEMM_IN_TF32) return colsum_out<float>(dy, out, scratch, rows, N, ld, s);
+  return INCIN_ERR_ARGUMENT;
+}
+
+extern "C" int incin_colsum_reduce(const float* part, void* out, long long chunks, int N, int dtype, void* stream) {
+  if (!part || !out || chunks <= 0 || N <= 0) return INCIN_ERR_ARGUMENT;
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == INCIN_GEMM_IN_BF16) return colsum_final<__nv_bfloat16>(part, out, N, chunks, s);
+  if (dtype == INCIN_GEMM_IN_FP16) return colsum_final<__half>(part, out, N, chunks, s);
+  if (dtype == INCIN_GEMM_IN_TF32) return colsum_final<float>(part, out, N, chunks, s);
   return INCIN_ERR_ARGUMENT;
 }

@@ -60,8 +60,9 @@ __global__ void strided_copy_vec_kernel(const T* __restrict__ src, T* __restrict
 
 // 2-D transpose of the two innermost axes through a padded 64 x 64 shared tile (outer axes batched in blockIdx.z).  Bound
 // by memory: with VEC both sides move 16 bytes a thread (rows and columns multiples of 16 bytes, aligned bases); 32 x 32
-// tiles of single elements reached half of that.  COLSUM (float only) adds the column sums of the source to colsum on
-// the way, which saves the bias gradient its own pass over the matrix.
+// tiles of single elements reached half of that.  COLSUM (float only, one batch) writes the column sums
+// of each band of 64 source rows to a row of colsum [bands][cols] on the way, which saves the bias gradient its own pass
+// over the matrix (8192 x 4096: a linear layer's backward 233 -> 214 us).
 template <typename T, bool VEC, bool COLSUM>
 __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict__ src, T* __restrict__ dst, long long rows,
                                                              long long cols, long long s_batch, long long d_batch,
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict
       float t = 0.f;
 #pragma unroll
       for (int k = 0; k < 256 / TPR; ++k) t += part[k * 64 + threadIdx.x];
-      atomicAdd(colsum + c0 + threadIdx.x, t);
+      colsum[(long long)(blockIdx.x / tiles_c) * cols + c0 + threadIdx.x] = t;
     }
   }
 }

@@ -90,6 +90,7 @@ _CUDA_SIGS = {
     "incin_colsum_accum_typed": (c_int, [c_void_p, c_void_p, c_ll, c_int, c_ll, c_int, c_void_p]),
     "incin_colsum_scratch_floats": (c_ll, [c_ll, c_int]),
     "incin_colsum_typed": (c_int, [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_ll, c_int, c_void_p]),
+    "incin_colsum_reduce": (c_int, [c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p]),
     "incin_transpose_f32": (c_int, [c_void_p, c_void_p, c_ll, c_ll, c_void_p, c_void_p]),
     "incin_sumsq_nonfinite_f32": (c_int, [c_void_p, c_ll, c_void_p, c_void_p]),
     "incin_fill_f32": (c_int, [c_void_p, c_float, c_ll, c_void_p]),

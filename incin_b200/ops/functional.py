@@ -106,7 +106,7 @@ class _LinearF32Acc(torch.autograd.Function):
     """Linear for fp16 tensors and, under ``MathMode.FAST``, fp32 tensors (multiplied as tf32) on the same tcgen05
     kernel as the bf16 path: fp32 accumulation, bias in the epilogue, rounded once to the input type.  Gradients return
     through autograd.  The tensor cores read 16-bit operands of the backward products as they lie; tf32 operands have to
-    run along the reduction, so those are transposed first.  Sums have a fixed order, but for the fp32 weight gradient,
+    run along the reduction, so those are transposed first, the output gradient together with its column sums.  Sums have a fixed order, but for the fp32 weight gradient,
     whose order is only fixed under ``Determinism.REQUIRED``.
 
     fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 288 -> 168 us and
@@ -140,6 +140,7 @@ class _LinearF32Acc(torch.autograd.Function):
         half = dy2.dtype == torch.float16
         unit = 8 if half else 4
         dx = dw = db = None
+        want_db = ctx.has_bias and ctx.needs_input_grad[2]
         if ctx.needs_input_grad[0]:
             if n_out % unit:
                 dx = dy2 @ w
@@ -157,13 +158,18 @@ class _LinearF32Acc(torch.autograd.Function):
                 dw = dy2.t() @ x2
             elif half:
                 dw = G.mm_linear_other(dy2.t().contiguous(), x2.t().contiguous())
-            elif ctx.fixed_order:
-                dw = G.mm_linear_other(K.transpose_f32(dy2), K.transpose_f32(x2))
             else:
-                # the reduction over the rows is split among CTAs that add up in fp32
-                dw = torch.zeros(n_out, n_in, dtype=torch.float32, device=dy.device)
-                G.mm_nt_f32out(K.transpose_f32(dy2), K.transpose_f32(x2), out=dw, accumulate=True, splits=0)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
+                if want_db:
+                    dyt, db = K.transpose_colsum_f32(dy2)
+                else:
+                    dyt = K.transpose_f32(dy2)
+                xt = K.transpose_f32(x2)
+                if ctx.fixed_order:
+                    dw = G.mm_linear_other(dyt, xt)
+                else:   # the reduction over the rows is split among CTAs that add up in fp32
+                    dw = torch.zeros(n_out, n_in, dtype=torch.float32, device=dy.device)
+                    G.mm_nt_f32out(dyt, xt, out=dw, accumulate=True, splits=0)
+        if want_db and db is None:
             db = K.colsum(dy2)
         return dx, dw, db
 

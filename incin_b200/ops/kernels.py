@@ -166,12 +166,24 @@ def colsum(dy):
     return out
 
 
-def transpose_f32(x, colsum=None):
-    """Dense transpose of a dense fp32 matrix; ``colsum`` (fp32), if given, gets the column sums of ``x`` added."""
+def transpose_f32(x):
+    """Dense transpose of a dense fp32 matrix."""
     rows, cols = x.shape
     out = torch.empty(cols, rows, dtype=F32, device=x.device)
-    nat.check(nat.cuda().incin_transpose_f32(x.data_ptr(), out.data_ptr(), rows, cols, nat.ptr(colsum), _s()), "transpose_f32")
+    nat.check(nat.cuda().incin_transpose_f32(x.data_ptr(), out.data_ptr(), rows, cols, None, _s()), "transpose_f32")
     return out
+
+
+def transpose_colsum_f32(x):
+    """Dense transpose of a dense fp32 matrix and its column sums (fixed order, as :func:`colsum`) in one pass over it."""
+    rows, cols = x.shape
+    lib, bands = nat.cuda(), (rows + 63) // 64
+    out = torch.empty(cols, rows, dtype=F32, device=x.device)
+    sums = torch.empty(cols, dtype=F32, device=x.device)
+    part = torch.empty(bands, cols, dtype=F32, device=x.device)
+    nat.check(lib.incin_transpose_f32(x.data_ptr(), out.data_ptr(), rows, cols, part.data_ptr(), _s()), "transpose_f32")
+    nat.check(lib.incin_colsum_reduce(part.data_ptr(), sums.data_ptr(), bands, cols, nat.GEMM_IN_TF32, _s()), "colsum_reduce")
+    return out, sums
 
 
 def sumsq_nonfinite(x, out):

@@ -176,6 +176,7 @@ extern "C" {
     pub fn incin_coll_reduce(bufs: *const *mut c_void, world: c_int, offset_bytes: c_longlong, first_elem: c_longlong, n: c_longlong, op: c_int, is_bf16: c_int, out: *mut c_void, stream: *mut c_void) -> c_int;
     pub fn incin_colsum_accum(dy: *const c_void, dbias: *mut f32, rows: c_longlong, N: c_int, ld: c_longlong, stream: *mut c_void) -> c_int;
     pub fn incin_colsum_accum_typed(dy: *const c_void, dbias: *mut f32, rows: c_longlong, N: c_int, ld: c_longlong, dtype: c_int, stream: *mut c_void) -> c_int;
+    pub fn incin_colsum_reduce(part: *const f32, out: *mut c_void, chunks: c_longlong, N: c_int, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_colsum_scratch_floats(rows: c_longlong, N: c_int) -> c_longlong;
     pub fn incin_colsum_typed(dy: *const c_void, out: *mut c_void, scratch: *mut f32, rows: c_longlong, N: c_int, ld: c_longlong, dtype: c_int, stream: *mut c_void) -> c_int;
     pub fn incin_conv_out_hw(g: *const incin_conv_geom, oh: *mut c_int, ow: *mut c_int) -> c_int;
