@@ -135,6 +135,8 @@ class _LinearF32Acc(torch.autograd.Function):
     def backward(ctx, dy):
         x2, w = ctx.saved_tensors
         dy2 = _c(dy).reshape(-1, dy.shape[-1])
+        if dy2.data_ptr() % 16:   # a view that starts inside a buffer: the products want 16-byte rows
+            dy2 = dy2.clone()
         rows, n_out = dy2.shape
         n_in = x2.shape[1]
         half = dy2.dtype == torch.float16
@@ -151,7 +153,7 @@ class _LinearF32Acc(torch.autograd.Function):
                 dx = G.mm_linear_other(dy2, K.transpose_f32(_c(w)))
             dx = dx.reshape(ctx.shape)
         if ctx.needs_input_grad[1]:
-            if half and n_out % unit == 0 and dy2.data_ptr() % 16 == 0:
+            if half and n_out % unit == 0:
                 dw = torch.empty(n_out, n_in, dtype=w.dtype, device=dy.device)
                 G.gemm(dy2, x2, dw, M=n_out, N=n_in, K=rows, lda=n_out, ldb=n_in, ldc=n_in, a_mn=True, b_mn=True)
             elif rows % unit:

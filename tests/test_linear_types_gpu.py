@@ -81,6 +81,26 @@ def test_linear_gradients_repeat(dtype, rows, n_in, n_out):
     assert ((first[2].double() - ref).abs() <= 2.0 ** -11 * ref.abs() * (dtype == torch.float16) + 2.0 ** -18 * dy.double().abs().sum(0)).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("rows,n_in,n_out", [(64, 32, 40), (7, 16, 12), (9, 24, 33)])
+@pytest.mark.parametrize("wanted", [(0, 1, 2), (0,), (1,), (2,)])
+def test_linear_unaligned_output_gradient(dtype, rows, n_in, n_out, wanted):
+    """An output gradient that starts one element into a buffer gives the same gradients as an aligned copy of it."""
+    from incin_b200.core.policy import Determinism, MathMode, policy_scope
+    from incin_b200.ops import functional as F
+    g = torch.Generator().manual_seed(rows)
+    x, w, b, dy = (torch.randn(*s, generator=g).to(dtype).cuda() for s in ((rows, n_in), (n_out, n_in), (n_out,), (rows, n_out)))
+    leaves = [t.requires_grad_(i in wanted) for i, t in enumerate((x, w, b))]
+    shifted = torch.zeros(dy.numel() + 1, dtype=dtype, device="cuda")
+    shifted[1:] = dy.reshape(-1)
+    got = []
+    for d in (dy, shifted[1:].view_as(dy)):
+        with policy_scope(math=MathMode.FAST, determinism=Determinism.REQUIRED):
+            y = F.linear(x, w, b)
+        got.append(torch.autograd.grad(y, [leaves[i] for i in wanted], d))
+    assert all(torch.equal(p, q) for p, q in zip(*got))
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
 @pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48), (1, 4194400, 1), (1, 1, 4194500)])
 def test_transpose_tiles(dtype, batch, rows, cols):
