@@ -28,6 +28,28 @@ struct ConvGeom {
   int N, C, H, W, KH, KW, OH, OW, sh, sw, ph, pw, dh, dw;
 };
 
+// A divisor known before the launch.  I, here and below, is the type of a flat index: 32 bits wherever the tensor has fewer
+// than 2^31 elements, and then a quotient is one multiplication, because dividing (64-bit indices above all) was most of the
+// time of these kernels.  With 2^(s - 1) < d <= 2^s and mul = ceil(2^(31 + s) / d), which is below 2^32, mul * d exceeds
+// 2^(31 + s) by less than 2^s, so n * mul / 2^(31 + s) exceeds n / d by less than 1 / d for n < 2^31: the floors agree.
+template <typename I>
+struct Divisor {
+  I d;
+  explicit Divisor(long long v) : d((I)v) {}
+  __device__ __forceinline__ I of(I n) const { return n / d; }
+};
+template <>
+struct Divisor<unsigned> {
+  unsigned d, mul;
+  int shift = 31;
+  explicit Divisor(long long v) : d((unsigned)v) {
+    while (shift < 62 && (1ull << (shift - 31)) < d) ++shift;
+    mul = (unsigned)(((1ull << shift) + d - 1) / d);
+  }
+  __device__ __forceinline__ unsigned of(unsigned n) const { return (unsigned)(((unsigned long long)n * mul) >> shift); }
+};
+using Div = Divisor<unsigned>;   // of values below 2^31
+
 // cols[(n*OH+oh)*OW+ow][(c*KH+kh)*KW+kw] = x[n][c][oh*sh-ph+kh*dh][ow*sw-pw+kw*dw] (0 outside)
 template <typename T>
 __global__ void im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, long long total) {
@@ -188,81 +210,64 @@ __global__ void __launch_bounds__(256) col2im_tile_kernel(const T* __restrict__ 
 }
 
 // ---- pooling ---------------------------------------------------------------------------------------------------
-// The rows of all planes, walked by groups of blockDim.x threads (8, 16 or 32: the width decides, so that narrow planes
-// do not idle most of a warp): plane and row advance by fixed steps, and nothing is divided inside the loop.
-struct RowWalk {
-  long long plane, plane_step, r, r_step, rows;
-  int i, i_step, height;
-  __device__ __forceinline__ RowWalk(long long rows_, int height_) {
-    rows = rows_;
-    height = height_;
-    r = (long long)blockIdx.x * blockDim.y + threadIdx.y;
-    r_step = (long long)gridDim.x * blockDim.y;
-    plane = r / height;
-    i = (int)(r - plane * height);
-    plane_step = r_step / height;
-    i_step = (int)(r_step - plane_step * height);
-  }
-  __device__ __forceinline__ bool more() const { return r < rows; }
-  __device__ __forceinline__ void next() {
-    r += r_step;
-    plane += plane_step;
-    i += i_step;
-    if (i >= height) {
-      i -= height;
-      ++plane;
-    }
+// One thread an element, whatever the shape of a plane
+template <typename I>
+struct Place {
+  int x, y;
+  long long plane;
+  __device__ __forceinline__ Place(I t, const Divisor<I>& width, const Divisor<I>& height) {
+    const I row = width.of(t), p = height.of(row);
+    x = (int)(t - row * width.d);
+    y = (int)(row - p * height.d);
+    plane = (long long)p;
   }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) maxpool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int* __restrict__ arg, ConvGeom g,
-                                                          long long rows) {
-  for (RowWalk w(rows, g.OH); w.more(); w.next()) {
-    const int oh = w.i;
-    const T* p = x + w.plane * g.H * g.W;
-    for (int ow = threadIdx.x; ow < g.OW; ow += blockDim.x) {
-      float best = -INFINITY;
-      int best_i = -1;
-      for (int kh = 0; kh < g.KH; ++kh) {
-        const int ih = oh * g.sh - g.ph + kh;
-        if (ih < 0 || ih >= g.H) continue;
-        for (int kw = 0; kw < g.KW; ++kw) {
-          const int iw = ow * g.sw - g.pw + kw;
-          if (iw < 0 || iw >= g.W) continue;
-          const float v = ldf(p, (long long)ih * g.W + iw);
-          if (v > best || v != v || best_i < 0) {
-            best = v;
-            best_i = ih * g.W + iw;
-          }
+template <typename T, typename I>
+__global__ void maxpool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int* __restrict__ arg, ConvGeom g, I total, Divisor<I> OW, Divisor<I> OH) {
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const Place<I> o(t, OW, OH);
+    const T* p = x + o.plane * g.H * g.W;
+    float best = -INFINITY;
+    int best_i = -1;
+    for (int kh = 0; kh < g.KH; ++kh) {
+      const int ih = o.y * g.sh - g.ph + kh;
+      if (ih < 0 || ih >= g.H) continue;
+      for (int kw = 0; kw < g.KW; ++kw) {
+        const int iw = o.x * g.sw - g.pw + kw;
+        if (iw < 0 || iw >= g.W) continue;
+        const float v = ldf(p, (long long)ih * g.W + iw);
+        if (v > best || v != v || best_i < 0) {
+          best = v;
+          best_i = ih * g.W + iw;
         }
       }
-      stf(y, w.r * g.OW + ow, best);
-      if (arg) arg[w.r * g.OW + ow] = best_i;
     }
+    stf(y, (long long)t, best);
+    if (arg) arg[t] = best_i;
   }
 }
 
 // dx[plane][i] = sum of dy over the windows whose argmax is i: gather over the windows that cover pixel i (N 64, C 64,
-// 32 x 32 bf16, 2 x 2 windows: 38 -> 26 us; with a 64-bit index split per pixel the divisions were most of it)
-template <typename T>
-__global__ void __launch_bounds__(256) maxpool_bwd_kernel(const T* __restrict__ dy, const int* __restrict__ arg, T* __restrict__ dx, ConvGeom g,
-                                                          long long rows) {
-  for (int iw = threadIdx.x; iw < g.W; iw += blockDim.x) {
-    const int ow_lo = max(0, (iw + g.pw - g.KW + g.sw) / g.sw), ow_hi = min(g.OW - 1, (iw + g.pw) / g.sw);
-    for (RowWalk w(rows, g.H); w.more(); w.next()) {
-      const int ih = w.i, me = ih * g.W + iw;
-      const int oh_lo = max(0, (ih + g.ph - g.KH + g.sh) / g.sh), oh_hi = min(g.OH - 1, (ih + g.ph) / g.sh);
-      const T* dyp = dy + w.plane * g.OH * g.OW;
-      const int* ap = arg + w.plane * g.OH * g.OW;
-      float acc = 0.0f;
-      for (int oh = oh_lo; oh <= oh_hi; ++oh)
-        for (int ow = ow_lo; ow <= ow_hi; ++ow) {
-          const long long o = (long long)oh * g.OW + ow;
-          if (ap[o] == me) acc += ldf(dyp, o);
-        }
-      stf(dx, w.r * g.W + iw, acc);
-    }
+// 32 x 32 bf16, 2 x 2 windows: 38 us with divisions of 64-bit indices -> 20; a row at a time per group of threads took 25
+// there and 24 ms on one row of 10^6)
+template <typename T, typename I>
+__global__ void maxpool_bwd_kernel(const T* __restrict__ dy, const int* __restrict__ arg, T* __restrict__ dx, ConvGeom g, I total,
+                                   Divisor<I> W, Divisor<I> H, Div SH, Div SW) {
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const Place<I> i(t, W, H);
+    const int me = i.y * g.W + i.x;
+    const int oh_lo = (int)SH.of((unsigned)max(0, i.y + g.ph - g.KH + g.sh)), oh_hi = min(g.OH - 1, (int)SH.of((unsigned)(i.y + g.ph)));
+    const int ow_lo = (int)SW.of((unsigned)max(0, i.x + g.pw - g.KW + g.sw)), ow_hi = min(g.OW - 1, (int)SW.of((unsigned)(i.x + g.pw)));
+    const T* dyp = dy + i.plane * g.OH * g.OW;
+    const int* ap = arg + i.plane * g.OH * g.OW;
+    float acc = 0.0f;
+    for (int oh = oh_lo; oh <= oh_hi; ++oh)
+      for (int ow = ow_lo; ow <= ow_hi; ++ow) {
+        const long long o = (long long)oh * g.OW + ow;
+        if (ap[o] == me) acc += ldf(dyp, o);
+      }
+    stf(dx, (long long)t, acc);
   }
 }
 
@@ -459,76 +464,45 @@ __global__ void __launch_bounds__(512) batchnorm_bwd_kernel(const T* __restrict_
 // ---- adaptive average pooling: output cell (oh, ow) averages rows [floor(oh*H/OH), ceil((oh+1)*H/OH)) x the same in w
 // (crates/incin-backends/src/cuda/ops/kernels/pool.cu adaptive_avg_pool2d_{fwd,bwd}; the backward there scatters with
 // atomics, here every input pixel gathers from the output cells whose window contains it)
-// (quotients of products that fit 32 bits are taken in 32 bits: a 64-bit division costs several times as much)
-__device__ __forceinline__ int ad_div(long long a, int b) {
-  return a <= 0x7fffffffLL ? (int)((unsigned)a / (unsigned)b) : (int)(a / b);
+// (products below 2^31 are divided in 32 bits)
+__device__ __forceinline__ int ad_div(long long a, const Div& b) {
+  return a <= 0x7fffffffLL ? (int)b.of((unsigned)a) : (int)(a / b.d);
 }
-__device__ __forceinline__ int ad_start(int o, int in, int out) { return ad_div((long long)o * in, out); }
-__device__ __forceinline__ int ad_end(int o, int in, int out) { return ad_div(((long long)o + 1) * in + out - 1, out); }
+__device__ __forceinline__ int ad_start(int o, int in, const Div& out) { return ad_div((long long)o * in, out); }
+__device__ __forceinline__ int ad_end(int o, int in, const Div& out) { return ad_div(((long long)o + 1) * in + out.d - 1, out); }
 
-template <typename T>
-__global__ void adaptive_avgpool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, int H, int W, int OH, int OW, long long total) {
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int ow = (int)(t % OW), oh = (int)((t / OW) % OH);
-    const long long plane = t / ((long long)OW * OH);
-    const int h0 = ad_start(oh, H, OH), h1 = ad_end(oh, H, OH), w0 = ad_start(ow, W, OW), w1 = ad_end(ow, W, OW);
-    const T* p = x + plane * H * W;
+template <typename T, typename I>
+__global__ void adaptive_avgpool_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, Div H, Div W, Div OH, Div OW, I total, Divisor<I> oh_,
+                                            Divisor<I> ow_) {
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const Place<I> o(t, ow_, oh_);
+    const int h0 = ad_start(o.y, H.d, OH), h1 = ad_end(o.y, H.d, OH), w0 = ad_start(o.x, W.d, OW), w1 = ad_end(o.x, W.d, OW);
+    const T* p = x + o.plane * H.d * W.d;
     float acc = 0.0f;
     for (int h = h0; h < h1; ++h)
-      for (int w = w0; w < w1; ++w) acc += ldf(p, (long long)h * W + w);
-    stf(y, t, acc / (float)((h1 - h0) * (w1 - w0)));
+      for (int w = w0; w < w1; ++w) acc += ldf(p, (long long)h * W.d + w);
+    stf(y, (long long)t, acc / (float)((h1 - h0) * (w1 - w0)));
   }
 }
 
-// Output cells that contain an input index, and their extents, along one axis: cell o covers [start(o), end(o)).  The
-// cells of index i are neighbours (lo .. hi - 1).
-struct CellRange {
-  int lo, hi;
-};
-__device__ __forceinline__ CellRange cells_of(int i, int in, int out) {
-  CellRange r;
-  r.lo = ad_div((long long)i * out, in);
-  r.hi = ad_div(((long long)i + 1) * out + in - 1, in);
-  while (r.lo > 0 && ad_end(r.lo - 1, in, out) > i) --r.lo;
-  while (r.hi < out && ad_start(r.hi, in, out) <= i) ++r.hi;
-  while (r.lo < r.hi && ad_end(r.lo, in, out) <= i) ++r.lo;           // only cells that do contain i
-  while (r.hi > r.lo && ad_start(r.hi - 1, in, out) > i) --r.hi;
-  return r;
-}
-
-// TAB: a block first tabulates the cells of every row and column index and the extent of every cell (the host has checked
-// that they fit the table), so that a pixel costs table reads and one division by the area.  Without the table the
-// quotients are worked out per pixel.  N 64, C 128, 16 x 16 -> 4 x 4 bf16: 48 -> 26 us.
-constexpr int kCellTable = 1024;
-template <typename T, bool TAB>
-__global__ void __launch_bounds__(256) adaptive_avgpool_bwd_kernel(const T* __restrict__ dy, T* __restrict__ dx, int H, int W, int OH, int OW,
-                                                                   long long rows) {
-  __shared__ CellRange tab_h[TAB ? kCellTable : 1], tab_w[TAB ? kCellTable : 1];
-  __shared__ int ext_h[TAB ? kCellTable : 1], ext_w[TAB ? kCellTable : 1];
-  if constexpr (TAB) {
-    for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < kCellTable; i += blockDim.x * blockDim.y) {
-      if (i < H) tab_h[i] = cells_of(i, H, OH);
-      if (i < W) tab_w[i] = cells_of(i, W, OW);
-      if (i < OH) ext_h[i] = ad_end(i, H, OH) - ad_start(i, H, OH);
-      if (i < OW) ext_w[i] = ad_end(i, W, OW) - ad_start(i, W, OW);
-    }
-    __syncthreads();
-  }
-  for (RowWalk k(rows, H); k.more(); k.next()) {
-    const T* p = dy + k.plane * OH * OW;
-    const CellRange rh = TAB ? tab_h[k.i] : cells_of(k.i, H, OH);
-    for (int w = threadIdx.x; w < W; w += blockDim.x) {
-      const CellRange rw = TAB ? tab_w[w] : cells_of(w, W, OW);
-      float acc = 0.0f;
-      for (int oh = rh.lo; oh < rh.hi; ++oh) {
-        const int eh = TAB ? ext_h[oh] : ad_end(oh, H, OH) - ad_start(oh, H, OH);
-        for (int ow = rw.lo; ow < rw.hi; ++ow) {
-          const int ew = TAB ? ext_w[ow] : ad_end(ow, W, OW) - ad_start(ow, W, OW);
-          acc += ldf(p, (long long)oh * OW + ow) / (float)(eh * ew);
-        }
+// Input index i lies in cell o, [start(o), end(o)), if and only if o * in < (i + 1) * out and (o + 1) * in > i * out: the
+// cells floor(i * out / in) .. ceil((i + 1) * out / in) - 1.  N 64, C 128, 16 x 16 -> 4 x 4 bf16: 47 -> 20 us.
+template <typename T, typename I>
+__global__ void adaptive_avgpool_bwd_kernel(const T* __restrict__ dy, T* __restrict__ dx, Div H, Div W, Div OH, Div OW, I total, Divisor<I> h_,
+                                            Divisor<I> w_) {
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const Place<I> i(t, w_, h_);
+    const T* p = dy + i.plane * OH.d * OW.d;
+    const int oh_lo = ad_start(i.y, OH.d, H), oh_hi = ad_end(i.y, OH.d, H), ow_lo = ad_start(i.x, OW.d, W), ow_hi = ad_end(i.x, OW.d, W);
+    float acc = 0.0f;
+    for (int oh = oh_lo; oh < oh_hi; ++oh) {
+      const int eh = ad_end(oh, H.d, OH) - ad_start(oh, H.d, OH);
+      for (int ow = ow_lo; ow < ow_hi; ++ow) {
+        const int ew = ad_end(ow, W.d, OW) - ad_start(ow, W.d, OW);
+        acc += ldf(p, (long long)oh * OW.d + ow) / (float)(eh * ew);
       }
-      stf(dx, k.r * W + w, acc);
     }
+    stf(dx, (long long)t, acc);
   }
 }
 
@@ -537,14 +511,10 @@ inline unsigned grid_for(long long n) {
   return (unsigned)(g < 1 ? 1 : (g > 148LL * 16 ? 148LL * 16 : g));
 }
 
-// launch shape of the kernels that walk rows: a row's threads by rows, 256 together, and up to 16 blocks an SM
-inline dim3 row_block(int width) {
-  const unsigned x = width > 16 ? 32 : (width > 8 ? 16 : 8);
-  return dim3(x, 256 / x);
-}
-inline unsigned row_grid(long long rows, int width) {
-  const long long per = row_block(width).y, b = (rows + per - 1) / per;
-  return (unsigned)(b < 1 ? 1 : (b > 148LL * 16 ? 148LL * 16 : b));
+// calls f with the element count in the narrowest type that the kernels' flat index can have (a step past the end fits too)
+template <typename F> void with_index(long long total, F f) {
+  if (total < 0x7fffffffLL) f((unsigned)total);
+  else f(total);
 }
 
 ConvGeom geom(const incin_conv_geom* d) {
@@ -660,24 +630,33 @@ extern "C" int incin_col2im(const void* cols, void* dx, const incin_conv_geom* d
   return is_bf16 ? col2im_t<__nv_bfloat16>(cols, dx, geom(d), s) : col2im_t<float>(cols, dx, geom(d), s);
 }
 
+template <typename T>
+static void maxpool_fwd_t(const void* x, void* y, int* argmax, const ConvGeom& g, cudaStream_t s) {
+  with_index((long long)g.N * g.C * g.OH * g.OW, [&](auto total) {
+    maxpool_fwd_kernel<T><<<grid_for((long long)total), 256, 0, s>>>(static_cast<const T*>(x), static_cast<T*>(y), argmax, g, total,
+                                                                  Divisor<decltype(total)>(g.OW), Divisor<decltype(total)>(g.OH));
+  });
+}
+template <typename T>
+static void maxpool_bwd_t(const void* dy, const int* argmax, void* dx, const ConvGeom& g, cudaStream_t s) {
+  with_index((long long)g.N * g.C * g.H * g.W, [&](auto total) {
+    maxpool_bwd_kernel<T><<<grid_for((long long)total), 256, 0, s>>>(static_cast<const T*>(dy), argmax, static_cast<T*>(dx), g, total,
+                                                                  Divisor<decltype(total)>(g.W), Divisor<decltype(total)>(g.H), Div(g.sh), Div(g.sw));
+  });
+}
+
 extern "C" int incin_maxpool2d_fwd(const void* x, void* y, int* argmax, const incin_conv_geom* d, int is_bf16, void* stream) {
   if (!x || !y || !valid(d)) return INCIN_ERR_ARGUMENT;
-  const ConvGeom g = geom(d);
-  const long long total = (long long)g.N * g.C * g.OH;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  DISPATCH(is_bf16, (maxpool_fwd_kernel<__nv_bfloat16><<<row_grid(total, g.OW), row_block(g.OW), 0, s>>>(static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), argmax, g, total)),
-           (maxpool_fwd_kernel<float><<<row_grid(total, g.OW), row_block(g.OW), 0, s>>>(static_cast<const float*>(x), static_cast<float*>(y), argmax, g, total)));
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  DISPATCH(is_bf16, maxpool_fwd_t<__nv_bfloat16>(x, y, argmax, geom(d), s), maxpool_fwd_t<float>(x, y, argmax, geom(d), s));
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
 extern "C" int incin_maxpool2d_bwd(const void* dy, const int* argmax, void* dx, const incin_conv_geom* d, int is_bf16,
                                    void* stream) {
   if (!dy || !argmax || !dx || !valid(d)) return INCIN_ERR_ARGUMENT;
-  const ConvGeom g = geom(d);
-  const long long total = (long long)g.N * g.C * g.H;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  DISPATCH(is_bf16, (maxpool_bwd_kernel<__nv_bfloat16><<<row_grid(total, g.W), row_block(g.W), 0, s>>>(static_cast<const __nv_bfloat16*>(dy), argmax, static_cast<__nv_bfloat16*>(dx), g, total)),
-           (maxpool_bwd_kernel<float><<<row_grid(total, g.W), row_block(g.W), 0, s>>>(static_cast<const float*>(dy), argmax, static_cast<float*>(dx), g, total)));
+  const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  DISPATCH(is_bf16, maxpool_bwd_t<__nv_bfloat16>(dy, argmax, dx, geom(d), s), maxpool_bwd_t<float>(dy, argmax, dx, geom(d), s));
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
@@ -750,17 +729,17 @@ extern "C" int incin_adaptive_avgpool2d(const void* in, void* out, long long pla
   if (!in || !out || planes <= 0 || H <= 0 || W <= 0 || OH <= 0 || OW <= 0) return INCIN_ERR_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
   const long long total = planes * (backward ? (long long)H * W : (long long)OH * OW);
-  if (backward) {
-    const bool tab = H <= kCellTable && W <= kCellTable && OH <= kCellTable && OW <= kCellTable;
-    const long long rows = planes * H;
-    auto go = [&](auto kern, auto* dy, auto* dx) { kern<<<row_grid(rows, W), row_block(W), 0, s>>>(dy, dx, H, W, OH, OW, rows); };
-    DISPATCH(is_bf16,
-             (go(tab ? adaptive_avgpool_bwd_kernel<__nv_bfloat16, true> : adaptive_avgpool_bwd_kernel<__nv_bfloat16, false>, (const __nv_bfloat16*)in, (__nv_bfloat16*)out)),
-             (go(tab ? adaptive_avgpool_bwd_kernel<float, true> : adaptive_avgpool_bwd_kernel<float, false>, (const float*)in, (float*)out)));
-  }
-  else
-    DISPATCH(is_bf16,
-             (adaptive_avgpool_fwd_kernel<<<grid_for(total), 256, 0, s>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, H, W, OH, OW, total)),
-             (adaptive_avgpool_fwd_kernel<<<grid_for(total), 256, 0, s>>>((const float*)in, (float*)out, H, W, OH, OW, total)));
+  const Div h(H), w(W), oh(OH), ow(OW);
+  with_index(total, [&](auto n) {
+    using I = decltype(n);
+    if (backward)
+      DISPATCH(is_bf16,
+               (adaptive_avgpool_bwd_kernel<<<grid_for(total), 256, 0, s>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, h, w, oh, ow, n, Divisor<I>(H), Divisor<I>(W))),
+               (adaptive_avgpool_bwd_kernel<<<grid_for(total), 256, 0, s>>>((const float*)in, (float*)out, h, w, oh, ow, n, Divisor<I>(H), Divisor<I>(W))));
+    else
+      DISPATCH(is_bf16,
+               (adaptive_avgpool_fwd_kernel<<<grid_for(total), 256, 0, s>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, h, w, oh, ow, n, Divisor<I>(OH), Divisor<I>(OW))),
+               (adaptive_avgpool_fwd_kernel<<<grid_for(total), 256, 0, s>>>((const float*)in, (float*)out, h, w, oh, ow, n, Divisor<I>(OH), Divisor<I>(OW))));
+  });
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }

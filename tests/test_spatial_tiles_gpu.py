@@ -1,4 +1,4 @@
-"""Tiled convolution helpers, cluster batch norm and row-mapped pooling at the sizes where their tiles end."""
+"""Tiled convolution helpers, cluster batch norm and pooling at the sizes where their tiles end."""
 import pytest
 import torch
 import torch.nn.functional as TF
@@ -58,8 +58,9 @@ def test_batch_norm_slices(dtype, shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("shape,k,s,p", [((1, 1, 1, 1), 1, 1, 0), ((3, 5, 7, 33), 3, 2, 1), ((2, 9, 8, 8), 2, 2, 0), ((2, 3, 40, 65), (3, 2), (1, 3), (1, 0))])
-def test_max_pool_rows(dtype, shape, k, s, p):
+@pytest.mark.parametrize("shape,k,s,p", [((1, 1, 1, 1), 1, 1, 0), ((3, 5, 7, 33), 3, 2, 1), ((2, 9, 8, 8), 2, 2, 0), ((2, 3, 40, 65), (3, 2), (1, 3), (1, 0)),
+                                         ((1, 2, 1, 70001), (1, 3), (1, 2), (0, 1)), ((2, 1, 30001, 1), (2, 1), (2, 1), (0, 0))])
+def test_max_pool_shapes(dtype, shape, k, s, p):
     from incin_b200.ops import tensor_ops as T
     g = torch.Generator().manual_seed(shape[-1])
     x = torch.randn(shape, generator=g).to(dtype).cuda().requires_grad_()
@@ -68,6 +69,23 @@ def test_max_pool_rows(dtype, shape, k, s, p):
     assert torch.equal(y.float(), yr)
     dy = torch.randint(-2, 3, y.shape, generator=g).to(dtype).cuda()
     assert torch.equal(torch.autograd.grad(y, x, dy)[0].float(), torch.autograd.grad(yr, xr, dy.float())[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("planes,hw,out", [((2, 3), (7, 5), (3, 2)), ((1, 4), (5, 7), (8, 9)), ((3, 1), (1, 50001), (1, 7)), ((2, 2), (40, 1), (6, 1)),
+                                           ((2, 8), (16, 16), (4, 4)), ((1, 1), (1, 1), (1, 1)), ((1, 2), (1, 9), (1, 4000))])
+def test_adaptive_pool_shapes(dtype, planes, hw, out):
+    from incin_b200.ops import tensor_ops as T
+    g = torch.Generator().manual_seed(hw[1])
+    x = torch.randn(*planes, *hw, generator=g).to(dtype).cuda().requires_grad_()
+    xd = x.detach().double().requires_grad_()
+    y, yd = T.adaptive_avg_pool2d(x, out), TF.adaptive_avg_pool2d(xd, out)
+    dy = torch.randn(y.shape, generator=g).to(dtype).cuda()
+    dx, dxd = torch.autograd.grad(y, x, dy)[0], torch.autograd.grad(yd, xd, dy.double())[0]
+    # fp32 sums of up to in / out or out / in terms, quotients of 2^-22 (--use_fast_math), one rounding to the type
+    u = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -21
+    for got, ref in ((y, yd), (dx, dxd)):
+        assert ((got.double() - ref).abs() <= u * ref.abs() + 2.0 ** -16 * ref.abs().max() + 1e-7).all()
 
 
 @pytest.mark.parametrize("perm", [(0, 2, 3, 1), (0, 3, 1, 2), (1, 0, 2, 3), (3, 2, 1, 0)])
