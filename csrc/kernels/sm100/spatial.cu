@@ -6,12 +6,13 @@
 //   * im2col writes the [N*OH*OW, C*KH*KW] matrix the tcgen05 GEMM consumes directly (K-major rows), and col2im
 //     GATHERS the contributions of each input pixel, so the data gradient needs no atomics and is deterministic;
 //   * max pooling keeps the argmax (int32 offset inside the plane) so its backward is a gather as well;
-//   * batch norm has a training forward (per-channel mean / biased variance in one pass over the channel with a
-//     block per channel, running statistics updated in the same kernel) and a full backward.
+//   * batch norm has a training forward (per-channel mean / biased variance in one pass over the channel with
+//     one CTA or a small cluster per channel, running statistics updated in the same kernel) and a full backward.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cooperative_groups.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "incin_b200.h"
 
@@ -300,7 +301,7 @@ __global__ void avgpool_kernel(const T* __restrict__ in, T* __restrict__ out, Co
   }
 }
 
-// ---- batch norm (one block per channel) -------------------------------------------------------------------------
+// ---- batch norm (a block, or a cluster of up to eight, per channel) -------------------------------------------------------------------------
 __device__ __forceinline__ float2 block_sum2(float a, float b) {
   __shared__ float sa[32], sb[32];
 #pragma unroll
@@ -322,11 +323,14 @@ __device__ __forceinline__ float2 block_sum2(float a, float b) {
   return make_float2(ra, rb);
 }
 
-// Training forward and backward: a thread-block cluster of 1 to 8 CTAs per channel, whose partial sums meet in
+// Training forward and backward: one CTA per channel, or (CL) a thread-block cluster of 2 to 8, whose partial sums meet in
 // distributed shared memory (fixed order, so results repeat to the bit).  The two passes over the channel are the work;
 // one CTA per channel left most SMs idle at 64 to 128 channels and split a 64-bit index per element.  With VEC 16 bytes
 // are read and written at a time (HW a multiple of that, aligned bases).  N 64, C 64, 32 x 32 and
-// N 64, C 128, 16 x 16 in bf16, average: forward 53 -> 9.5 us, backward 60 -> 10 us.
+// N 64, C 128, 16 x 16 in bf16, average: forward 53 -> 9.5 us, backward 60 -> 10 us.  Channels of one CTA do without the
+// cluster and its barriers, and short ones (fewer than 512 16-byte pieces, a piece a thread) take an element a thread:
+// (one cluster kernel for all | this) N 32, C 4096, HW 4 forward 30 -> 17 us, backward 46 -> 27; N 2, C 1000, HW 64 10.1 -> 6.1 and
+// 14.8 -> 10.9.
 __device__ __forceinline__ float2 cluster_sum2(float2 mine) {
   __shared__ float2 part;
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -346,6 +350,7 @@ __device__ __forceinline__ float2 cluster_sum2(float2 mine) {
 template <int V, typename I, typename F>
 __device__ __forceinline__ void channel_loop(int N, int C, long long HW, int c, int slice, int slices, F f) {
   const I hwv = (I)(HW / V), count = (I)N * hwv;
+#pragma unroll V == 1 ? 4 : 1
   for (I i = (I)slice * blockDim.x + threadIdx.x; i < count; i += (I)slices * blockDim.x) {
     const I n = i / hwv, j = i - n * hwv;
     f(((long long)n * C + c) * HW + (long long)j * V);
@@ -366,13 +371,13 @@ template <int V, typename T> __device__ __forceinline__ void store_v(T* p, const
   else p[0] = e[0];
 }
 
-template <typename T, int V, typename I>
+template <bool CL, typename T, int V, typename I>
 __global__ void __launch_bounds__(512) batchnorm_train_fwd_kernel(const T* __restrict__ x, const float* __restrict__ gamma,
                                                                   const float* __restrict__ beta, T* __restrict__ y,
                                                                   float* __restrict__ save_mean, float* __restrict__ save_rstd,
                                                                   float* __restrict__ run_mean, float* __restrict__ run_var, int N, int C,
                                                                   long long HW, float eps, float momentum) {
-  const int slices = (int)cooperative_groups::this_cluster().num_blocks();
+  const int slices = CL ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
   const int c = blockIdx.x / slices, slice = blockIdx.x % slices;
   const long long count = (long long)N * HW;
   // shifted sums (shift = first element of the channel) keep the one-pass variance accurate for large means
@@ -388,7 +393,8 @@ __global__ void __launch_bounds__(512) batchnorm_train_fwd_kernel(const T* __res
       ss += d * d;
     }
   });
-  const float2 r = cluster_sum2(block_sum2(s, ss));
+  float2 r = block_sum2(s, ss);
+  if constexpr (CL) r = cluster_sum2(r);
   const float m_sh = r.x / (float)count;
   const float var = fmaxf(r.y / (float)count - m_sh * m_sh, 0.0f);
   const float mean = m_sh + shift, rstd = rsqrtf(var + eps);
@@ -420,13 +426,13 @@ __global__ void batchnorm_eval_kernel(const T* __restrict__ x, const float* __re
 }
 
 // dx = gamma*rstd/M * (M*dy - sum(dy) - xhat*sum(dy*xhat)); dgamma += sum(dy*xhat); dbeta += sum(dy)
-template <typename T, int V, typename I>
+template <bool CL, typename T, int V, typename I>
 __global__ void __launch_bounds__(512) batchnorm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x,
                                                             const float* __restrict__ gamma, const float* __restrict__ save_mean,
                                                             const float* __restrict__ save_rstd, T* __restrict__ dx,
                                                             float* __restrict__ dgamma, float* __restrict__ dbeta, int N, int C,
                                                             long long HW) {
-  const int slices = (int)cooperative_groups::this_cluster().num_blocks();
+  const int slices = CL ? (int)cooperative_groups::this_cluster().num_blocks() : 1;
   const int c = blockIdx.x / slices, slice = blockIdx.x % slices;
   const long long count = (long long)N * HW;
   const float mean = save_mean[c], rstd = save_rstd[c];
@@ -441,7 +447,8 @@ __global__ void __launch_bounds__(512) batchnorm_bwd_kernel(const T* __restrict_
       s2 += g[k] * (v[k] - mean) * rstd;
     }
   });
-  const float2 r = cluster_sum2(block_sum2(s1, s2));
+  float2 r = block_sum2(s1, s2);
+  if constexpr (CL) r = cluster_sum2(r);
   if (threadIdx.x == 0 && slice == 0) {
     if (dgamma) dgamma[c] += r.y;
     if (dbeta) dbeta[c] += r.x;
@@ -535,7 +542,6 @@ bool valid(const incin_conv_geom* d) {
 
 }  // namespace
 
-// One cluster of `slices` CTAs per channel: enough CTAs for four on every SM, at least 4096 elements each, 8 at most.
 template <typename... KArgs, typename... Args>
 static int launch_channels(void (*kern)(KArgs...), int C, int slices, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -548,10 +554,11 @@ static int launch_channels(void (*kern)(KArgs...), int C, int slices, cudaStream
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = slices > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess && cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
+// CTAs per channel: enough for four on every SM, at least 4096 elements each, 8 at most
 static int channel_slices(long long C, long long count) {
   int s = 1;
   while (s < 8 && C * s < 4 * 148 && count / (2 * s) >= 4096) s *= 2;
@@ -676,10 +683,15 @@ static int batchnorm_train_fwd_t(const void* x, const float* gamma, const float*
                                  cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   const long long count = (long long)N * HW;
-  const bool vec = HW % V == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
-  auto kern = count > 0x40000000LL ? batchnorm_train_fwd_kernel<T, 1, long long>
-                                   : (vec ? batchnorm_train_fwd_kernel<T, V, unsigned> : batchnorm_train_fwd_kernel<T, 1, unsigned>);
-  return launch_channels(kern, C, channel_slices(C, count), s, static_cast<const T*>(x), gamma, beta, static_cast<T*>(y), save_mean,
+  const bool vec = HW % V == 0 && count >= 512 * V && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  const int slices = channel_slices(C, count);
+  auto pick = [&](auto cl) {
+    constexpr bool CL = decltype(cl)::value;
+    return count > 0x40000000LL ? batchnorm_train_fwd_kernel<CL, T, 1, long long>
+                                : (vec ? batchnorm_train_fwd_kernel<CL, T, V, unsigned> : batchnorm_train_fwd_kernel<CL, T, 1, unsigned>);
+  };
+  auto kern = slices > 1 ? pick(std::true_type{}) : pick(std::false_type{});
+  return launch_channels(kern, C, slices, s, static_cast<const T*>(x), gamma, beta, static_cast<T*>(y), save_mean,
                          save_rstd, running_mean, running_var, N, C, HW, eps, momentum);
 }
 
@@ -688,11 +700,16 @@ static int batchnorm_bwd_t(const void* dy, const void* x, const float* gamma, co
                            float* dgamma, float* dbeta, int N, int C, long long HW, cudaStream_t s) {
   constexpr int V = 16 / sizeof(T);
   const long long count = (long long)N * HW;
-  const bool vec = HW % V == 0 &&
+  const bool vec = HW % V == 0 && count >= 512 * V &&
                    ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0;
-  auto kern = count > 0x40000000LL ? batchnorm_bwd_kernel<T, 1, long long>
-                                   : (vec ? batchnorm_bwd_kernel<T, V, unsigned> : batchnorm_bwd_kernel<T, 1, unsigned>);
-  return launch_channels(kern, C, channel_slices(C, count), s, static_cast<const T*>(dy), static_cast<const T*>(x), gamma, save_mean,
+  const int slices = channel_slices(C, count);
+  auto pick = [&](auto cl) {
+    constexpr bool CL = decltype(cl)::value;
+    return count > 0x40000000LL ? batchnorm_bwd_kernel<CL, T, 1, long long>
+                                : (vec ? batchnorm_bwd_kernel<CL, T, V, unsigned> : batchnorm_bwd_kernel<CL, T, 1, unsigned>);
+  };
+  auto kern = slices > 1 ? pick(std::true_type{}) : pick(std::false_type{});
+  return launch_channels(kern, C, slices, s, static_cast<const T*>(dy), static_cast<const T*>(x), gamma, save_mean,
                          save_rstd, static_cast<T*>(dx), dgamma, dbeta, N, C, HW);
 }
 
