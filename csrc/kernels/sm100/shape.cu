@@ -58,23 +58,22 @@ __global__ void strided_copy_vec_kernel(const T* __restrict__ src, T* __restrict
   }
 }
 
-// 2-D transpose of the two innermost axes through a padded 64 x 64 shared tile (outer axes batched in blockIdx.z).  Bound
-// by memory: with VEC both sides move 16 bytes a thread (rows and columns multiples of 16 bytes, aligned bases); 32 x 32
-// tiles of single elements reached half of that.  COLSUM (float only, one batch) writes the column sums
+// 2-D transpose of the two innermost axes through a padded TS x TS shared tile (outer axes batched in blockIdx.z).  Bound
+// by memory: with V > 1 both sides move V elements, 16 bytes, a thread (rows and columns multiples of V, aligned bases);
+// 32 x 32 tiles of single elements reached half of that.  COLSUM (float only, one batch) writes the column sums
 // of each band of 64 source rows to a row of colsum [bands][cols] on the way, which saves the bias gradient its own pass
 // over the matrix (8192 x 4096: a linear layer's backward 233 -> 214 us).
-template <typename T, bool VEC, bool COLSUM>
+template <typename T, int TS, int V, bool COLSUM>
 __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict__ src, T* __restrict__ dst, long long rows,
                                                              long long cols, long long s_batch, long long d_batch,
                                                              float* __restrict__ colsum) {
-  constexpr int V = VEC ? 16 / (int)sizeof(T) : 1;   // elements per access
-  constexpr int TPR = 64 / V;                        // threads per row of the tile
-  constexpr int PITCH = sizeof(T) == 2 ? 66 : 65;    // 2-byte rows start 33 words apart: no bank conflicts on the way in
-  __shared__ T tile[64 * PITCH];
+  constexpr int TPR = TS / V;                          // threads per row of the tile
+  constexpr int PITCH = sizeof(T) == 2 ? TS + 2 : TS + 1;   // 2-byte rows start 33 words apart: no bank conflicts on the way in
+  __shared__ T tile[TS * PITCH];
   const T* s = src + blockIdx.z * s_batch;
   T* d = dst + blockIdx.z * d_batch;
-  const unsigned tiles_c = (unsigned)((cols + 63) / 64);   // column tiles fastest, in one grid axis: no limit on either side
-  const long long c0 = (long long)(blockIdx.x % tiles_c) * 64, r0 = (long long)(blockIdx.x / tiles_c) * 64;
+  const unsigned tiles_c = (unsigned)((cols + TS - 1) / TS);   // column tiles fastest, in one grid axis: no limit on either side
+  const long long c0 = (long long)(blockIdx.x % tiles_c) * TS, r0 = (long long)(blockIdx.x / tiles_c) * TS;
   const int tv = (threadIdx.x % TPR) * V, tr = threadIdx.x / TPR;
   float sum[V];
   if constexpr (COLSUM) {
@@ -82,11 +81,11 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict
     for (int k = 0; k < V; ++k) sum[k] = 0.f;
   }
 #pragma unroll
-  for (int j = tr; j < 64; j += 256 / TPR) {
+  for (int j = tr; j < TS; j += 256 / TPR) {
     const long long r = r0 + j, c = c0 + tv;
     if (r < rows && c < cols) {
       alignas(16) T e[V];
-      if constexpr (VEC) *reinterpret_cast<uint4*>(e) = *reinterpret_cast<const uint4*>(s + r * cols + c);
+      if constexpr (V > 1) *reinterpret_cast<uint4*>(e) = *reinterpret_cast<const uint4*>(s + r * cols + c);
       else e[0] = s[r * cols + c];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
@@ -97,13 +96,13 @@ __global__ void __launch_bounds__(256) transpose_tile_kernel(const T* __restrict
   }
   __syncthreads();
 #pragma unroll
-  for (int j = tr; j < 64; j += 256 / TPR) {
+  for (int j = tr; j < TS; j += 256 / TPR) {
     const long long c = c0 + j, r = r0 + tv;
     if (r < rows && c < cols) {
       alignas(16) T e[V];
 #pragma unroll
       for (int k = 0; k < V; ++k) e[k] = tile[(tv + k) * PITCH + j];
-      if constexpr (VEC) *reinterpret_cast<uint4*>(d + c * rows + r) = *reinterpret_cast<const uint4*>(e);
+      if constexpr (V > 1) *reinterpret_cast<uint4*>(d + c * rows + r) = *reinterpret_cast<const uint4*>(e);
       else d[c * rows + r] = e[0];
     }
   }
@@ -221,14 +220,24 @@ inline unsigned grid_for(long long n, int block) {
 }
 
 // src [batch, rows, cols] -> dst [batch, cols, rows], both dense; at most 65535 batches and 2^31 - 1 tiles each
-inline long long transpose_tiles(long long rows, long long cols) { return ((rows + 63) / 64) * ((cols + 63) / 64); }
+inline long long transpose_tiles(long long rows, long long cols, int ts = 64) { return ((rows + ts - 1) / ts) * ((cols + ts - 1) / ts); }
+template <typename T>
+bool transpose_vec(const T* src, const T* dst, long long rows, long long cols) {
+  constexpr int V = 16 / sizeof(T);
+  return V > 1 && rows % V == 0 && cols % V == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+}
 template <typename T, bool COLSUM>
 int transpose_launch(const T* src, T* dst, long long rows, long long cols, long long batch, float* colsum, cudaStream_t s) {
+  auto go = [&](auto kern, int ts) {
+    kern<<<dim3((unsigned)transpose_tiles(rows, cols, ts), 1, (unsigned)batch), 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
+  };
   constexpr int V = 16 / sizeof(T);
-  const dim3 grid((unsigned)transpose_tiles(rows, cols), 1, (unsigned)batch);
-  const bool vec = rows % V == 0 && cols % V == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-  if (vec) transpose_tile_kernel<T, true, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
-  else transpose_tile_kernel<T, false, COLSUM><<<grid, 256, 0, s>>>(src, dst, rows, cols, rows * cols, rows * cols, colsum);
+  constexpr int TS = sizeof(T) == 8 ? 32 : 64;   // pairs of 8 bytes conflict in 64 columns: 4096 x 4096 52 us, in 32 42
+  // Fewer than two tiles per SM: sixteen rounds of single accesses are the time, so small tiles (333 x 1001 bf16 3.6 -> 2.6 us)
+  const bool small = !COLSUM && transpose_tiles(rows, cols) * batch < 2 * 148;
+  if (transpose_vec(src, dst, rows, cols)) go(transpose_tile_kernel<T, TS, V, COLSUM>, TS);
+  else if (small) go(transpose_tile_kernel<T, 32, 1, false>, 32);
+  else go(transpose_tile_kernel<T, 64, 1, COLSUM>, 64);
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
 
@@ -244,9 +253,16 @@ int strided_copy_t(const void* src, void* dst, const Geometry& g, cudaStream_t s
       g.sstride[last - 1] == 1 && g.sstride[last] == g.shape[last - 1]) {
     const long long rows = g.shape[last], cols = g.shape[last - 1];   // source is [.., rows(last), cols(last-1)] dense
     const long long batch = g.rank == 3 ? g.shape[0] : 1;
-    if (batch <= 65535 && transpose_tiles(rows, cols) <= 0x7fffffffLL && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols))) {
-      return transpose_launch<T, false>(static_cast<const T*>(src), static_cast<T*>(dst), rows, cols, batch, nullptr, s);
-    }
+    const T *from = static_cast<const T*>(src);
+    T *to = static_cast<T*>(dst);
+    const long long tiles = transpose_tiles(rows, cols);
+    const bool v = transpose_vec(from, to, rows, cols);
+    // A tile costs the same however little of it is used (0.9 ns over the whole GPU in pieces of eight elements, 4.9 ns one
+    // by one), an element of the general copy 5.5 ps: thin matrices go there.  [32, 3, 224, 224] -> channels last 108 -> 27 us,
+    // 60000 of 4 x 4 210 -> 8 us, 4000 of 10 x 128 39 -> 28 us; against it 20000 of 40 x 24 27 us, 99 in the general copy.
+    const bool filled = rows * cols >= tiles * (v ? 64 + 576 / VEC : 896) || (!v && tiles * batch < 2 * 148);
+    if (filled && batch <= 65535 && transpose_tiles(rows, cols, 32) <= 0x7fffffffLL && (g.rank == 2 || (g.sstride[0] == rows * cols && g.dstride[0] == rows * cols)))
+      return transpose_launch<T, false>(from, to, rows, cols, batch, nullptr, s);
   }
   bool vec = g.sstride[last] == 1 && g.dstride[last] == 1 && g.shape[last] % VEC == 0 &&
              ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;

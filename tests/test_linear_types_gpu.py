@@ -102,7 +102,8 @@ def test_linear_unaligned_output_gradient(dtype, rows, n_in, n_out, wanted):
 
 
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.float64])
-@pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48), (1, 4194400, 1), (1, 1, 4194500)])
+@pytest.mark.parametrize("batch,rows,cols", [(1, 1, 1), (1, 64, 64), (3, 63, 65), (2, 128, 80), (1, 1, 300), (2, 144, 48), (1, 4194400, 1), (1, 1, 4194500),
+                                             (300, 5, 7), (300, 16, 8), (5, 10, 128), (1, 333, 1001), (1, 2000, 1040), (700, 40, 24)])
 def test_transpose_tiles(dtype, batch, rows, cols):
     from incin_b200.ops import tensor_ops as T
     g = torch.Generator().manual_seed(rows)
