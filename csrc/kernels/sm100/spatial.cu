@@ -52,17 +52,17 @@ struct Divisor<unsigned> {
 using Div = Divisor<unsigned>;   // of values below 2^31
 
 // cols[(n*OH+oh)*OW+ow][(c*KH+kh)*KW+kw] = x[n][c][oh*sh-ph+kh*dh][ow*sw-pw+kw*dw] (0 outside)
-template <typename T>
-__global__ void im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, long long total) {
-  const int K = g.C * g.KH * g.KW;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(t % K);
-    const long long row = t / K;
-    const int ow = (int)(row % g.OW), oh = (int)((row / g.OW) % g.OH), n = (int)(row / ((long long)g.OW * g.OH));
-    const int kw = k % g.KW, kh = (k / g.KW) % g.KH, c = k / (g.KW * g.KH);
+template <typename T, typename I>
+__global__ void im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, I total, Divisor<I> K, Divisor<I> OW, Divisor<I> OH,
+                              Div KW, Div KH) {
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const I row = K.of(t), line = OW.of(row), image = OH.of(line);
+    const unsigned k = (unsigned)(t - row * K.d), q = KW.of(k);
+    const int ow = (int)(row - line * OW.d), oh = (int)(line - image * OH.d);
+    const int c = (int)KH.of(q), kw = (int)(k - q * KW.d), kh = (int)q - c * g.KH;
     const int ih = oh * g.sh - g.ph + kh * g.dh, iw = ow * g.sw - g.pw + kw * g.dw;
     T v = T(0.0f);
-    if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) v = x[(((long long)n * g.C + c) * g.H + ih) * g.W + iw];
+    if (ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) v = x[(((long long)image * g.C + c) * g.H + ih) * g.W + iw];
     cols[t] = v;
   }
 }
@@ -72,7 +72,7 @@ __global__ void im2col_kernel(const T* __restrict__ x, T* __restrict__ cols, Con
 // matrix from them.  tab[k] is where element k of the block's channels lies for ow = 0, so the inner loop has no index
 // arithmetic.  A warp takes 2 units of a row by 16 output columns: whole sectors on the way out, few bank conflicts on
 // the way in.  Bound by the column matrix it writes (K / C times the input).  N 64, C 64, 3 x 3, bf16,
-// 32 x 32 and 16 x 16 together (75 and 19 MB): 390 -> 70 us; the general kernel divides a 64-bit index per element.
+// 32 x 32 and 16 x 16 together (75 and 19 MB): 390 -> 70 us.
 template <typename T>
 __global__ void __launch_bounds__(256) im2col_tile_kernel(const T* __restrict__ x, T* __restrict__ cols, ConvGeom g, int CT, int SW) {
   extern __shared__ __align__(16) unsigned char im2col_smem[];
@@ -122,36 +122,39 @@ __global__ void __launch_bounds__(256) im2col_tile_kernel(const T* __restrict__ 
 }
 
 // dx[n][c][ih][iw] = sum over the (kh, kw, oh, ow) that read this pixel: a gather, no atomics
-template <typename T>
-__global__ void col2im_kernel(const T* __restrict__ cols, T* __restrict__ dx, ConvGeom g, long long total) {
+template <typename T, typename I>
+__global__ void col2im_kernel(const T* __restrict__ cols, T* __restrict__ dx, ConvGeom g, I total, Divisor<I> W, Divisor<I> H, Divisor<I> C,
+                              Div SH, Div SW) {
   const int K = g.C * g.KH * g.KW;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int iw = (int)(t % g.W), ih = (int)((t / g.W) % g.H);
-    const int c = (int)((t / ((long long)g.W * g.H)) % g.C), n = (int)(t / ((long long)g.W * g.H * g.C));
+  for (I t = (I)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (I)gridDim.x * blockDim.x) {
+    const I line = W.of(t), plane = H.of(line), image = C.of(plane);
+    const int iw = (int)(t - line * W.d), ih = (int)(line - plane * H.d), c = (int)(plane - image * C.d);
+    const T* from = cols + (long long)image * g.OH * g.OW * K;
     float acc = 0.0f;
     for (int kh = 0; kh < g.KH; ++kh) {
       const int hh = ih + g.ph - kh * g.dh;
-      if (hh < 0 || hh % g.sh) continue;
-      const int oh = hh / g.sh;
-      if (oh >= g.OH) continue;
+      if (hh < 0) continue;
+      const int oh = (int)SH.of((unsigned)hh);
+      if (oh * g.sh != hh || oh >= g.OH) continue;
       for (int kw = 0; kw < g.KW; ++kw) {
         const int ww = iw + g.pw - kw * g.dw;
-        if (ww < 0 || ww % g.sw) continue;
-        const int ow = ww / g.sw;
-        if (ow >= g.OW) continue;
-        acc += ldf(cols, (((long long)n * g.OH + oh) * g.OW + ow) * K + (c * g.KH + kh) * g.KW + kw);
+        if (ww < 0) continue;
+        const int ow = (int)SW.of((unsigned)ww);
+        if (ow * g.sw != ww || ow >= g.OW) continue;
+        acc += ldf(from, ((long long)oh * g.OW + ow) * K + (c * g.KH + kh) * g.KW + kw);
       }
     }
-    stf(dx, t, acc);
+    stf(dx, (long long)t, acc);
   }
 }
 
 // Tiled form.  A block owns RB input rows of CT channels of one image: the part of the column matrix that reaches them
 // (every output row that reads them, OW columns, CT * KH * KW elements) is staged in shared memory, 16 bytes a load, and
 // each thread gathers its pixels from there, in the same order of kh and kw as the general kernel.  The pitch is one
-// word more than the data, so that neighbouring pixels lie in different banks.  Bound by the column matrix it reads;
+// word more than the data, so that neighbouring pixels lie in different banks.  Strides of 1 only: with larger ones few of
+// the staged elements belong to a pixel's row (the dispatch has figures).  Bound by the column matrix it reads;
 // the same two layers: 191 -> 88 us.
-template <typename T, bool UNIT>   // UNIT: strides of 1, no divisions in the gather
+template <typename T>
 __global__ void __launch_bounds__(256) col2im_tile_kernel(const T* __restrict__ cols, T* __restrict__ dx, ConvGeom g, int CT, int RB) {
   extern __shared__ __align__(16) unsigned char col2im_smem[];
   constexpr int V = 16 / sizeof(T), WV = 4 / sizeof(T);               // elements per 16-byte load, per 4-byte word
@@ -160,8 +163,7 @@ __global__ void __launch_bounds__(256) col2im_tile_kernel(const T* __restrict__ 
   const int bands = (g.H + RB - 1) / RB;
   const int n = blockIdx.x / bands, i0 = (blockIdx.x % bands) * RB, i1 = min(i0 + RB, g.H);
   const int c0 = blockIdx.y * CT, nc = min(CT, g.C - c0), units = nc * KK / V;
-  const int lo = i0 + g.ph - (g.KH - 1) * g.dh;                       // output rows oh with lo <= oh * sh <= i1 - 1 + ph
-  const int oh0 = lo > 0 ? (lo + g.sh - 1) / g.sh : 0, oh1 = min(g.OH - 1, (i1 - 1 + g.ph) / g.sh);
+  const int oh0 = max(0, i0 + g.ph - (g.KH - 1) * g.dh), oh1 = min(g.OH - 1, i1 - 1 + g.ph);   // output rows that reach the band
   const long long K = (long long)g.C * KK;
   const T* src = cols + ((long long)n * g.OH + oh0) * g.OW * K + (long long)c0 * KK;
   const unsigned total = (unsigned)(max(0, oh1 - oh0 + 1) * g.OW * units);
@@ -192,16 +194,12 @@ __global__ void __launch_bounds__(256) col2im_tile_kernel(const T* __restrict__ 
     for (int iw = lane % lw; iw < g.W; iw += lw) {
       float acc = 0.0f;
       for (int kh = 0; kh < g.KH; ++kh) {
-        const int hh = ih + g.ph - kh * g.dh;
-        if (hh < 0 || (!UNIT && hh % g.sh)) continue;
-        const int oh = UNIT ? hh : hh / g.sh;
-        if (oh >= g.OH) continue;
+        const int oh = ih + g.ph - kh * g.dh;
+        if (oh < 0 || oh >= g.OH) continue;
         const T* line = tile + (oh - oh0) * g.OW * pitch + (c * g.KH + kh) * g.KW;
         for (int kw = 0; kw < g.KW; ++kw) {
-          const int ww = iw + g.pw - kw * g.dw;
-          if (ww < 0 || (!UNIT && ww % g.sw)) continue;
-          const int ow = UNIT ? ww : ww / g.sw;
-          if (ow >= g.OW) continue;
+          const int ow = iw + g.pw - kw * g.dw;
+          if (ow < 0 || ow >= g.OW) continue;
           acc += ldf(line, ow * pitch + kw);
         }
       }
@@ -592,12 +590,18 @@ static int im2col_t(const void* x, void* cols, const ConvGeom& g, cudaStream_t s
   const long long c8 = (g.C + 7) / 8 * 8;
   long long CT = 8;
   while (CT * 2 <= c8 && CT < 64 && bytes(CT * 2) <= kTileBytes / 2) CT *= 2;
-  if (g.C * KK % V == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 && KK <= 4096 && SW <= 65536 && bytes(CT) <= kTileBytes &&
+  // The tile pays where a row fills a warp's 16 columns and there is enough to write (bf16, tile | general: N 64, C 64, 32 x 32,
+  // 3 x 3 49 | 90 us; N 64, C 256, 8 x 8 37 | 25; N 1, C 64, 32 x 32 8.0 | 4.4; N 16, C 64, 8 x 8 patches 17 | 2.9).
+  if (g.OW >= 16 && total >= 3 << 19 && g.C * KK % V == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 && KK <= 4096 && SW <= 65536 && bytes(CT) <= kTileBytes &&
       (long long)g.N * g.OH <= 0x7fffffffLL && c8 / CT <= 65535) {
     const dim3 grid((unsigned)(g.N * g.OH), (unsigned)((g.C + CT - 1) / CT));
     im2col_tile_kernel<T><<<grid, 256, (size_t)bytes(CT), s>>>(static_cast<const T*>(x), static_cast<T*>(cols), g, (int)CT, (int)SW);
   } else {
-    im2col_kernel<T><<<grid_for(total), 256, 0, s>>>(static_cast<const T*>(x), static_cast<T*>(cols), g, total);
+    with_index(total, [&](auto n) {
+      using I = decltype(n);
+      im2col_kernel<T><<<grid_for(total), 256, 0, s>>>(static_cast<const T*>(x), static_cast<T*>(cols), g, n, Divisor<I>(g.C * KK), Divisor<I>(g.OW),
+                                                       Divisor<I>(g.OH), Div(g.KW), Div(g.KH));
+    });
   }
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }
@@ -607,20 +611,27 @@ static int col2im_t(const void* cols, void* dx, const ConvGeom& g, cudaStream_t 
   constexpr int V = 16 / sizeof(T), WV = 4 / sizeof(T), CT = 8;
   const long long KK = (long long)g.KH * g.KW, total = (long long)g.N * g.C * g.H * g.W;
   auto bytes = [&](long long rb) {   // output rows that reach rb input rows, at most
-    long long oh = (rb - 1 + (long long)(g.KH - 1) * g.dh) / g.sh + 1;
+    long long oh = rb + (long long)(g.KH - 1) * g.dh;
     if (oh > g.OH) oh = g.OH;
     return oh * g.OW * (CT * KK + WV) * (long long)sizeof(T);
   };
   long long RB = g.H < 8 ? g.H : 8;
   while (RB > 1 && bytes(RB) > kTileBytes) --RB;
   const long long bands = (g.H + RB - 1) / RB;
-  if (g.C * KK % V == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 && KK <= 4096 && bytes(RB) <= kTileBytes &&
-      g.N * bands <= 0x7fffffffLL && (g.C + CT - 1) / CT <= 65535) {
-    const dim3 grid((unsigned)(g.N * bands), (unsigned)((g.C + CT - 1) / CT));
-    auto kern = g.sh == 1 && g.sw == 1 ? col2im_tile_kernel<T, true> : col2im_tile_kernel<T, false>;
-    kern<<<grid, 256, (size_t)bytes(RB), s>>>(static_cast<const T*>(cols), static_cast<T*>(dx), g, CT, (int)RB);
+  const long long groups = (g.C + CT - 1) / CT;
+  // The tile pays where its rows are read KH times and there are blocks enough (bf16, tile | general: N 64, C 64, 32 x 32, 3 x 3
+  // 67 | 151 us; N 64, C 16, 14 x 14, 256 blocks, 9.6 | 7.1; N 8, C 16, 40 x 40, 128 blocks, 18 | 7.1; 1 x 1, N 8, C 256, 28 x 28
+  // 14 | 11).  Strides: 2 x 128 x 128, C 32, 3 x 3 by 4 42 | 10; 8 x 56 x 56, C 64, 3 x 3 by 2 51 | 25.
+  if (g.sh == 1 && g.sw == 1 && KK > 1 && g.N * bands * groups >= 256 && g.C * KK % V == 0 && (reinterpret_cast<uintptr_t>(cols) & 15) == 0 &&
+      KK <= 4096 && bytes(RB) <= kTileBytes && g.N * bands <= 0x7fffffffLL && groups <= 65535) {
+    const dim3 grid((unsigned)(g.N * bands), (unsigned)groups);
+    col2im_tile_kernel<T><<<grid, 256, (size_t)bytes(RB), s>>>(static_cast<const T*>(cols), static_cast<T*>(dx), g, CT, (int)RB);
   } else {
-    col2im_kernel<T><<<grid_for(total), 256, 0, s>>>(static_cast<const T*>(cols), static_cast<T*>(dx), g, total);
+    with_index(total, [&](auto n) {
+      using I = decltype(n);
+      col2im_kernel<T><<<grid_for(total), 256, 0, s>>>(static_cast<const T*>(cols), static_cast<T*>(dx), g, n, Divisor<I>(g.W), Divisor<I>(g.H),
+                                                       Divisor<I>(g.C), Div(g.sh), Div(g.sw));
+    });
   }
   return cudaGetLastError() == cudaSuccess ? INCIN_OK : INCIN_ERR_LAUNCH;
 }

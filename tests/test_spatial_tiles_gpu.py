@@ -16,6 +16,14 @@ pytestmark = pytest.mark.gpu
     (1, 8, 4, 3000, (3, 3), (1, 1), (1, 1), (1, 1)),      # does not fit at all: general kernels
     (2, 3, 10, 10, (3, 3), (1, 1), (1, 1), (1, 1)),       # K = 27: general kernels
     (2, 4, 6, 6, (2, 2), (3, 3), (0, 0), (1, 1)),         # pixels that no window reads
+    # large enough for the tiled kernels: odd lines, a half empty channel tile, dilation, one-row bands, strides, 1 x 1
+    (16, 64, 17, 33, (3, 3), (1, 1), (1, 1), (1, 1)),
+    (40, 24, 20, 21, (3, 3), (1, 1), (1, 1), (1, 1)),
+    (12, 40, 30, 19, (3, 3), (1, 1), (2, 2), (2, 2)),
+    (20, 16, 30, 90, (3, 3), (1, 1), (1, 1), (1, 1)),
+    (8, 40, 41, 50, (5, 3), (2, 1), (2, 0), (1, 2)),
+    (24, 72, 30, 31, (1, 1), (1, 1), (0, 0), (1, 1)),
+    (9, 64, 19, 17, (4, 4), (1, 1), (3, 3), (1, 1)),
 ])
 def test_im2col_col2im_tiles(dtype, N, C, H, W, k, s, p, d):
     from incin_b200.ops import tensor_ops as T
