@@ -267,26 +267,32 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long B, int T, i
   }
 }
 
-// The same for 16-byte aligned rows with D / 2 a multiple of 8 (at most ROPE_MAX_HALF).  A block takes ROPE_TOKENS
-// positions, works out their angles once for all heads (power, sine and cosine per pair and head were most of the general
-// kernel's time) and rotates eight pairs a thread with 16-byte accesses.  Bound by memory; 8192 positions, 36 heads of 64:
-// 57 -> 16 us.  Reads x and writes y (the same buffer for the in-place call); heads H .. Ht - 1 are copied, so that the
+// The same for 16-byte aligned rows with D / 2 a multiple of 8 (at most ROPE_MAX_HALF).  A block takes up to ROPE_TOKENS
+// positions, works out their angles once for all its heads (power, sine and cosine per pair and head were most of the
+// general kernel's time) and rotates eight pairs a thread with 16-byte accesses.  Bound by memory; 8192 positions, 36 heads
+// of 64: 57 -> 16 us.  Short calls are bound by their chain instead, so they get fewer positions a block, down to one, and
+// then fewer heads (out of place, always 8 positions a block -> this: 8 x 128 heads of 128 22.9 -> 3.7 us, 61 x 24 of 128
+// 8.5 -> 3.4 us; copy and general kernel 4.9 us both).
+// Reads x and writes y (the same buffer for the in-place call); heads H .. Ht - 1 are copied, so that the
 // caller who has to keep x does not copy it first (13 us there).
 constexpr int ROPE_TOKENS = 8, ROPE_MAX_HALF = 128;
 __global__ void __launch_bounds__(256) rope_vec_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, long long positions, int T, int H, int Ht,
-                                                       int D, long long sb, long long st, long long sh, float theta, int inverse) {
+                                                       int D, long long sb, long long st, long long sh, float theta, int inverse, int tokens,
+                                                       int heads) {
   pdl_launch_dependents();
   __shared__ float2 angle[ROPE_TOKENS * ROPE_MAX_HALF];
   const int half = D / 2, vecs = half / 8;
-  const long long first = (long long)blockIdx.x * ROPE_TOKENS;
-  const int n = (int)(positions - first < ROPE_TOKENS ? positions - first : ROPE_TOKENS);
-  for (int i = threadIdx.x; i < n * half; i += 256)
-    angle[i] = rope_angle((int)((first + i / half) % T), i % half, D, theta, inverse);
+  const long long first = (long long)blockIdx.x * tokens;
+  const int n = (int)(positions - first < tokens ? positions - first : tokens);
+  const int h0 = blockIdx.y * heads, nh = min(heads, Ht - h0);
+  if (h0 < H)
+    for (int i = threadIdx.x; i < n * half; i += 256)
+      angle[i] = rope_angle((int)((first + i / half) % T), i % half, D, theta, inverse);
   __syncthreads();
   pdl_wait();
-  const int per = Ht * vecs;
+  const int per = nh * vecs;
   for (int i = threadIdx.x; i < n * per; i += 256) {
-    const int tok = i / per, k = i - tok * per, h = k / vecs, v = k - h * vecs;
+    const int tok = i / per, k = i - tok * per, hk = k / vecs, v = k - hk * vecs, h = h0 + hk;
     const long long pos = first + tok, b = pos / T;
     const long long off = b * sb + (pos - b * T) * st + (long long)h * sh + v * 8;
     if (h >= H) {
@@ -455,23 +461,27 @@ static bool rope_vec_ok(long long positions, int heads, int D) {
   return D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && (positions + ROPE_TOKENS - 1) / ROPE_TOKENS <= 0x7fffffffLL &&
          (long long)heads * D <= (1 << 24);
 }
+static void rope_vec_launch(const void* x, void* y, long long positions, int T, int H, int Ht, int D, long long sb, long long st, long long sh,
+                            float theta, int inverse, cudaStream_t stream) {
+  int tokens = ROPE_TOKENS, heads = Ht;
+  while (tokens > 1 && positions < 2 * 148 * tokens) tokens /= 2;
+  const long long blocks = (positions + tokens - 1) / tokens;
+  while (heads > 1 && blocks * ((Ht + heads - 1) / heads) < 148 && (long long)tokens * heads * (D / 16) > 256) heads = (heads + 1) / 2;
+  launch_pdl(rope_vec_kernel, dim3((unsigned)blocks, (unsigned)((Ht + heads - 1) / heads)), dim3(256), 0, stream, (const __nv_bfloat16*)x,
+             (__nv_bfloat16*)y, positions, T, H, Ht, D, sb, st, sh, theta, inverse, tokens, heads);
+}
 extern "C" int incin_rope_out(const void* x, void* y, long long B, int T, int H, int Htot, int D, float theta, int inverse, void* stream) {
   if (!x || !y || B <= 0 || T <= 0 || H <= 0 || Htot < H || D <= 0 || (D & 1)) return INCIN_ERR_ARGUMENT;
-  const long long positions = B * T;
-  if (!rope_vec_ok(positions, Htot, D)) return INCIN_ERR_UNSUPPORTED;
+  if (!rope_vec_ok(B * T, Htot, D)) return INCIN_ERR_UNSUPPORTED;
   if (!vec16(x, y, y)) return INCIN_ERR_ALIGNMENT;
-  launch_pdl(rope_vec_kernel, dim3((unsigned)((positions + ROPE_TOKENS - 1) / ROPE_TOKENS)), dim3(256), 0, ST(stream),
-             (const __nv_bfloat16*)x, (__nv_bfloat16*)y, positions, T, H, Htot, D, (long long)T * Htot * D, (long long)Htot * D, (long long)D,
-             theta, inverse);
+  rope_vec_launch(x, y, B * T, T, H, Htot, D, (long long)T * Htot * D, (long long)Htot * D, D, theta, inverse, ST(stream));
   return CHECK_LAUNCH();
 }
 extern "C" int incin_rope(void* x, long long B, int T, int H, int D, long long stride_b, long long stride_t,
                           long long stride_h, float theta, int inverse, void* stream) {
   if (B <= 0 || T <= 0 || H <= 0 || D <= 0 || (D & 1)) return INCIN_ERR_ARGUMENT;
-  const long long positions = B * T, blocks = (positions + ROPE_TOKENS - 1) / ROPE_TOKENS;
-  if (rope_vec_ok(positions, H, D) && vec16(x, x, x) && stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0)
-    launch_pdl(rope_vec_kernel, dim3((unsigned)blocks), dim3(256), 0, ST(stream), (const __nv_bfloat16*)x, (__nv_bfloat16*)x, positions, T, H,
-               H, D, stride_b, stride_t, stride_h, theta, inverse);
+  if (rope_vec_ok(B * T, H, D) && vec16(x, x, x) && stride_b % 8 == 0 && stride_t % 8 == 0 && stride_h % 8 == 0)
+    rope_vec_launch(x, x, B * T, T, H, H, D, stride_b, stride_t, stride_h, theta, inverse, ST(stream));
   else
     launch_pdl(rope_kernel, dim3(grid_for(B * T * H * (D / 2), 256)), dim3(256), 0, ST(stream), (__nv_bfloat16*)x, B, T, H, D, stride_b,
                stride_t, stride_h, theta, inverse);

@@ -27,7 +27,8 @@ def test_swiglu(rows, F, shift):
 
 
 @pytest.mark.parametrize("inverse", [False, True])
-@pytest.mark.parametrize("B,T,H,D", [(1, 1, 1, 16), (2, 7, 3, 64), (3, 9, 4, 128), (1, 33, 2, 8), (2, 5, 2, 24), (1, 19, 36, 64), (2, 3, 1, 256)])
+@pytest.mark.parametrize("B,T,H,D", [(1, 1, 1, 16), (2, 7, 3, 64), (3, 9, 4, 128), (1, 33, 2, 8), (2, 5, 2, 24), (1, 19, 36, 64), (2, 3, 1, 256),
+                                     (1, 1, 126, 256), (1, 8, 125, 128), (3, 200, 3, 64), (1, 2500, 2, 32)])
 def test_rope(B, T, H, D, inverse):
     """Rotation of the first H of H + 2 heads in place; D / 2 no multiple of 8 takes the element-wise kernel."""
     from incin_b200.ops import kernels as K
