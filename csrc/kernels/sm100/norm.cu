@@ -466,7 +466,8 @@ norm_bwd_param_final(const float* __restrict__ scratch, float* __restrict__ dgam
 // in registers while the block walks its rows; the next row is requested before the block meets to add up the current
 // one.  Bound by memory: x, dy and dx_add read once, dx written.  The row-per-warp kernel read x and dy twice for dx and
 // the partial-sum kernel a third time.  8192 x 2048 RMS with dx_add: 54 -> 32 us with the final reduction
-// inside a training step, 66 -> 42 us with a cold L2; LayerNorm 65536 x 4096: 720 -> 509 us.
+// inside a training step, 66 -> 42 us with a cold L2; LayerNorm 65536 x 4096: 720 -> 509 us.  The block is as wide as the
+// row (160 threads up to 1280 columns: LayerNorm 32768 x 1032 102 -> 75 us, 141 with 256 threads and 222 blocks).
 // Block b takes rows b, b + gridDim.x, ... and writes scratch[b][{g}] (RMS) or scratch[b][{g, b}]; fixed order.
 __device__ __forceinline__ uint4 ld_row16(const __nv_bfloat16* p) {   // volatile: stays where the pipeline wants it
   uint4 v;
@@ -475,7 +476,7 @@ __device__ __forceinline__ uint4 ld_row16(const __nv_bfloat16* p) {   // volatil
 }
 
 template <bool RMS, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 3 : (THREADS == 384 ? 2 : 1))
+__global__ void __launch_bounds__(THREADS, THREADS <= 256 ? 3 : (THREADS == 384 ? 2 : 1))
 norm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gamma,
                      const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ dx_add,
                      __nv_bfloat16* dx, float* __restrict__ scratch, long long rows, int C) {
@@ -835,21 +836,23 @@ static int colsum_chunks(long long rows) {
 
 static bool wide_bwd_ok(int C) { return C > 1024 && C <= 4096 && C % 8 == 0; }
 
+static int two_pass_chunks(long long rows) {
+  const long long c = (rows + 127) / 128;
+  return (int)(c < 64 ? c : 64);
+}
+
 static int param_chunks(long long rows, int C) {
   if (fused_bwd_ok(C)) {
     const long long rp = fused_rows_per(rows, C);
     return (int)((rows + rp - 1) / rp);
   }
-  if (wide_bwd_ok(C)) {   // blocks of the one-pass kernel for LayerNorm; RMS has one sum per column and twice as many
+  if (wide_bwd_ok(C)) {   // blocks of the one-pass kernel: three per SM where the scratch allows it
     long long c = (1 << 19) / C;   // keeps the scratch within the 2^20 floats that callers without an allocator have
-    if (c > 222) c = 222;
+    if (c > 444) c = 444;
     if (c > rows) c = rows;
     return (int)c;
   }
-  long long c = (rows + 127) / 128;
-  if (c > 64) c = 64;
-  if (c < 1) c = 1;
-  return (int)c;
+  return two_pass_chunks(rows);
 }
 
 template <bool RMS>
@@ -891,15 +894,22 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
   }
   const bool aligned = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gamma) |
                          reinterpret_cast<uintptr_t>(dx_add) | reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0;
-  if (dgamma && wide_bwd_ok(C) && aligned) {
+  // The scratch leaves LayerNorm fewer than two blocks of 256 threads per SM from 1776 columns on, too few to fill the memory
+  // pipeline over many rows: 2048 columns, one pass | two: 2048 rows 14.7 | 19.3 us, 4096 22.2 | 27.2, 8192 50.8 | 48.2.
+  // (With 384 and 512 threads one block is enough: 8192 x 2560 54 | 66 us, 8192 x 4096 69 | 97.)
+  const bool starved = !RMS && C <= 2048 && rows > 4096 && param_chunks(rows, C) < 2 * 148;
+  if (dgamma && wide_bwd_ok(C) && aligned && !starved) {
     if (!scratch) return INCIN_ERR_ARGUMENT;
-    long long chunks = (long long)param_chunks(rows, C) * (RMS ? 2 : 1);
+    long long chunks = (long long)param_chunks(rows, C) * (RMS ? 2 : 1);   // (RMS has one sum per column)
+    if (chunks > 444) chunks = 444;
     if (chunks > rows) chunks = rows;
     auto go = [&](auto kern, int threads) {
       launch_pdl(kern, dim3((unsigned)chunks), dim3(threads), 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,
                  (const __nv_bfloat16*)gamma, mean, rstd, (const __nv_bfloat16*)dx_add, (__nv_bfloat16*)dx, scratch, rows, C);
     };
-    if (C <= 2048) go(norm_bwd_wide_kernel<RMS, 256>, 256);
+    if (C <= 1280) go(norm_bwd_wide_kernel<RMS, 160>, 160);
+    else if (C <= 1536) go(norm_bwd_wide_kernel<RMS, 192>, 192);
+    else if (C <= 2048) go(norm_bwd_wide_kernel<RMS, 256>, 256);
     else if (C <= 3072) go(norm_bwd_wide_kernel<RMS, 384>, 384);
     else go(norm_bwd_wide_kernel<RMS, 512>, 512);
     launch_pdl(norm_bwd_param_final, dim3((C + 31) / 32), dim3(32 * PF_LANES), 0, s, scratch, dgamma, dbeta, C, (int)chunks, RMS ? 1 : 2,
@@ -912,7 +922,7 @@ static int norm_bwd_launch(const void* dy, const void* x, const void* gamma, con
       (const __nv_bfloat16*)dx_add, (__nv_bfloat16*)dx, rows, C);
   if (dgamma) {
     if (!scratch) return INCIN_ERR_ARGUMENT;
-    const int chunks = param_chunks(rows, C);
+    const int chunks = two_pass_chunks(rows);
     if ((C % 8) == 0) {
       dim3 grid((C + 255) / 256, chunks);
       launch_pdl(norm_bwd_param_partial_vec<RMS>, dim3(grid), dim3(256), 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, mean,

@@ -6,7 +6,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rms", [True, False])
-@pytest.mark.parametrize("rows,C", [(1, 1032), (3, 2048), (700, 2048), (37, 2056), (5, 3072), (301, 3080), (150, 4096), (6, 4104), (9, 1100)])
+@pytest.mark.parametrize("rows,C", [(1, 1032), (3, 2048), (700, 2048), (37, 2056), (5, 3072), (301, 3080), (150, 4096), (6, 4104), (9, 1100),
+                                    (700, 1280), (445, 1288), (901, 1536), (30, 1544)])
 def test_norm_backward_wide(rms, rows, C):
     """Around the widths where the block size changes; 4104 and 1100 columns take the row-per-warp kernels."""
     from incin_b200.ops import kernels as K
