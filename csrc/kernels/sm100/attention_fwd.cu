@@ -408,6 +408,46 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
+}  // namespace incin
+
+#include "attention_fwd_tile.cuh"
+
+namespace incin {
+
+// Whether the kernel with one query tile per CTA is the faster one.  Measured over head_dim 64 and 128, 6 to 32 heads (grouped
+// and not), B 1 to 64, T 16 to 2048 (560 launches; the pairs alone are up to 1.8 times as slow at these, single tiles alone up
+// to 1.9 times at length).  Pairs | single tiles, in us:
+// - No more pairs than SMs: a pair takes longer than its two tiles side by side.  head_dim 128, B 1, H 8: T 64 5.6 | 4.3,
+//   T 192 8.7 | 6.1, T 300 9.4 | 8.1, T 384 9.5 | 9.9, T 448 12.0 | 10.5, T 1000 18.5 | 21.0.  At head_dim 64 only an even
+//   number of tiles loses (H 6: T 256 7.4 | 6.6, T 384 7.4 | 7.9, T 1000 15.8 | 14.2).  Where the single tiles do not fit
+//   the SMs at once either, the two are even, except at head_dim 128 up to T 192.
+// - More: both go in rounds, of a pair per SM and of two tiles per SM.  A pair of which only one tile exists counts as much
+//   as two, so with one or three tiles a head the rounds decide (H 12, D 64, T 128: B 16 8.3 | 7.1 in 2 | 1 rounds, B 32
+//   10.7 | 11.5 in 3 | 2); with two or five, how full the last one is (D 128, H 24 / 8, T 256: B 8 16.6 | 13.6 at 65 %,
+//   B 16 23.5 | 24.5 at 86 %).  At head_dim 128 single tiles stop after 64 keys: up to T 64 they always win (B 64, H 32:
+//   44.8 | 37.5), and gain more up to T 192 and T 320.
+static bool one_tile_per_cta(const incin_attn_desc* d, int sms) {
+  const int tiles = (d->T + FA_BM - 1) / FA_BM;
+  if (d->Hq > 65535 || d->B > 65535 || tiles > 65535) return false;   // its grid
+  const long long heads = (long long)d->Hq * d->B, pairs = (tiles + 1) / 2 * heads;
+  const bool wide = d->D == 128;
+  if (pairs <= sms) {
+    const bool half = pairs * 2 <= sms, third = pairs * 3 <= sms;
+    if (!wide) return tiles % 2 == 0 && (tiles <= 4 ? half : third);
+    return d->T <= 192 || (d->T <= 320 && half) || (d->T > 384 && d->T <= 448 && third);
+  }
+  if (wide && d->T <= 64) return true;
+  const long long rounds = (pairs + sms - 1) / sms, single_rounds = (tiles * heads + 2 * sms - 1) / (2 * sms);
+  auto emptier = [&](int percent) { return pairs * 100 < rounds * sms * percent; };   // than that, on average over the rounds
+  switch (tiles) {
+    case 1: return rounds <= 6 && rounds == 2 * single_rounds;
+    case 2: return wide && emptier(d->T <= 192 ? 87 : 75);
+    case 3: return 2 * rounds >= 3 * single_rounds || (wide && d->T <= 320 && emptier(87));
+    case 5: return emptier(75);
+    default: return false;
+  }
+}
+
 template <int D>
 static int launch_fwd(const incin_attn_desc* d, cudaStream_t stream) {
   using Cfg = FaCfg<D>;
@@ -454,7 +494,9 @@ extern "C" int incin_flash_attn_fwd(const incin_attn_desc* d, void* stream) {
     return INCIN_ERR_ARGUMENT;
   if ((d->o_stride_t % 8) || (d->o_stride_h % 8) || (d->o_stride_b % 8) || (reinterpret_cast<uintptr_t>(d->o) & 15))
     return INCIN_ERR_ALIGNMENT;
-  if (d->D == 64) return incin::launch_fwd<64>(d, (cudaStream_t)stream);
-  if (d->D == 128) return incin::launch_fwd<128>(d, (cudaStream_t)stream);
-  return INCIN_ERR_UNSUPPORTED;
+  if (d->D != 64 && d->D != 128) return INCIN_ERR_UNSUPPORTED;
+  const cudaStream_t s = (cudaStream_t)stream;
+  if (incin::one_tile_per_cta(d, incin::device_sm_count()))
+    return d->D == 64 ? incin::launch_fwd_tile<64, 128>(d, s) : incin::launch_fwd_tile<128, 64>(d, s);
+  return d->D == 64 ? incin::launch_fwd<64>(d, s) : incin::launch_fwd<128>(d, s);
 }

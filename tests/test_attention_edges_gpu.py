@@ -26,10 +26,12 @@ def test_backward_repeats_to_the_bit(B, T, H, D):
 
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 1, 1, 1), (2, 127, 3, 1), (1, 129, 2, 2), (3, 255, 2, 1), (1, 257, 4, 2),
-                                        (40, 384, 6, 2), (2, 1025, 5, 5)])
+                                        (40, 384, 6, 2), (2, 1025, 5, 5), (13, 128, 12, 4), (160, 64, 1, 1), (30, 192, 6, 6),
+                                        (10, 300, 16, 2), (5, 640, 20, 20), (64, 65, 12, 12)])
 def test_forward_tile_edges(B, T, Hq, Hkv, D):
-    """Query tiles come in pairs and items outnumber CTAs in some of these: one row, one tile, a pair with one tile
-    beyond the sequence, several items per CTA; strided inputs; rows whose scores need rescaling on every tile."""
+    """Both kernels (one tile per CTA where pairs of tiles would leave SMs idle).  Query tiles come in pairs and items
+    outnumber CTAs in some of these: one row, one tile, a pair with one tile beyond the sequence, several items per CTA;
+    strided inputs; rows whose scores need rescaling on every tile."""
     from incin_b200.ops import attention as A
     from incin_b200.ops import gemm as G
     g = torch.Generator().manual_seed(T + D)
@@ -49,6 +51,45 @@ def test_forward_tile_edges(B, T, Hq, Hkv, D):
     # |error| <= 2^-8 (sum p |v| + |o|), 5 % above it for the fp32 scores, exponentials and sums
     bound = 2.0 ** -8 * 1.05 * (torch.einsum("bhqk,bkhd->bqhd", p, vd.abs()) + ref.abs()) + 1e-5
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(8, 1000, 12, 12, 64), (2, 2000, 32, 4, 64), (2, 2000, 24, 8, 128), (2, 1665, 32, 32, 128),
+                                          (8, 300, 24, 8, 128), (13, 128, 12, 12, 64)])
+def test_forward_repeats_to_the_bit(B, T, Hq, Hkv, D):
+    """Every sum has a fixed order, so a product that starts before its operands are complete, or overwrites columns that
+    another one still reads, shows up as a difference."""
+    from incin_b200.ops import attention as A
+    from incin_b200.ops import gemm as G
+    g = torch.Generator().manual_seed(5)
+    q, k, v = (torch.randn(B, T, h, D, generator=g).to(torch.bfloat16).cuda() for h in (Hq, Hkv, Hkv))
+    with torch.no_grad():
+        first = A.flash_attention(q, k, v)
+        for _ in range(40):
+            assert torch.equal(A.flash_attention(q, k, v), first)
+    G.check_status()
+
+
+@pytest.mark.parametrize("B,T,Hq,Hkv,D", [(2, 1665, 32, 32, 128), (2, 1665, 64, 64, 64), (3, 2300, 40, 20, 128)])
+def test_forward_head_by_head(B, T, Hq, Hkv, D):
+    """K and V of more than 48 MB: the items are walked head by head.  Several items per CTA, an odd number of tiles."""
+    from incin_b200.ops import attention as A
+    from incin_b200.ops import gemm as G
+    assert B * Hkv * T * D * 4 > 48 << 20
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v = (torch.randn(B, T, h, D, generator=g, device="cuda").to(torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    with torch.no_grad():
+        out = A.flash_attention(q, k, v)
+    G.check_status()
+    mask = torch.ones(T, T, device="cuda", dtype=torch.bool).tril()
+    for b in range(B):
+        for h in range(0, Hq, 8):
+            heads = slice(h, h + 8)
+            kv = torch.arange(h, h + 8, device="cuda") // (Hq // Hkv)
+            qd, kd, vd = q[b, :, heads].double().transpose(0, 1), k[b, :, kv].double().transpose(0, 1), v[b, :, kv].double().transpose(0, 1)
+            p = torch.softmax((qd @ kd.mT * D ** -0.5).masked_fill(~mask, float("-inf")), -1)
+            ref = p @ vd
+            bound = 2.0 ** -8 * 1.05 * (p @ vd.abs() + ref.abs()) + 1e-5   # as in test_forward_tile_edges
+            assert ((out[b, :, heads].double().transpose(0, 1) - ref).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("B,T,Hq,Hkv", [(1, 900, 6, 2), (9, 384, 40, 40), (2, 1500, 16, 8)])
