@@ -447,10 +447,11 @@ __device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
 // Normal distribution function Phi(x) and e = exp(-x^2 / 2), for the erf form of GELU.
 // Phi(-|x|) = e * f(|x|) with f(a) = erfcx(a / sqrt 2) / 2, smooth and bounded, is a degree-6 polynomial in
 // s = p a / (1 + p a) in [0, 1) with constant term 1/2 (the variable is the classical one of rational erfc
-// approximations; coefficients fitted here for the least maximum error of Phi, 5.2e-9).  In fp32 arithmetic, against
-// 64 bits on N(0, 2^2) and [-12, 12]: gelu rms 4.5e-8, max 3.8e-7, gradient rms 2.5e-8, max 1.3e-7; with an exactly
-// rounded erf in x / 2 (1 + erf) 5.1e-8, 4.5e-7, 2.6e-8, 1.35e-7, and its tail (x < -3) loses all digits but two where
-// this keeps four.  Two special-function operations and 14 packed ones instead of a call with a branch: the GEMM
+// approximations; coefficients fitted here for the least maximum error of Phi, 6.0e-9 as they are rounded).  In fp32
+// arithmetic, against 64 bits on N(0, 2^2) and [-12, 12]: gelu rms 4.5e-8, max 3.8e-7, gradient rms 2.5e-8, max 1.3e-7; with
+// an exactly rounded erf in x / 2 (1 + erf) 5.1e-8, 4.5e-7, 2.6e-8, 1.35e-7.  Relative error of the tail, which that form
+// loses by cancellation from x = -3 on: 1.8e-6 down to x = -3, 1.5e-5 to -4, 7.7e-5 to -5, 2e-4 to -6, 6e-4 to -8 and
+// 1.6e-3 to -12.  Two special-function operations and 14 packed ones instead of a call with a branch: the GEMM
 // epilogues with GELU were bound by it (8192 x 768 -> 3072: with GELU and side output 59 -> 51 us, data gradient
 // with GELU' 88 -> 71 us; 35 us without).  |x| is capped where e has long vanished, so that infinities
 // do not meet 0 in s; NaN arrives through e.
