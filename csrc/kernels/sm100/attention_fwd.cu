@@ -13,13 +13,20 @@
 // O_w is only rescaled when the running max grew by more than 2^8 (the final division by the row sum makes the result
 // exact either way); the softmax threads do it themselves, with a tcgen05.ld / tcgen05.st round trip.
 //
+// The schedule (two query tiles in turn, rescaling only beyond 2^8, the second product started before all of P is there) is
+// that of the published FlashAttention-4.
+//
 // What bounds it: per 128 x 128 scores at head_dim 128 the tensor core needs 1024 clocks and the exponentials also 1024
-// (16 a clock and SM); at head_dim 64 512 against 1024.  Both units run at about 63 % (ncu): a tile's chain of loading, maximum,
-// exponentials and its two products is what is left over.  (2^x on the FMA pipe for a quarter of the scores changed
-// nothing, for more of them it was slower.)  One query tile per CTA with P through shared memory, two CTAs
-// per SM (the split before this one), made P's round trip and the wait for its product part of every tile's chain:
-// B 8, H 32, T 4096, D 128: 1505 -> 941 us (731 -> 1169 TFLOP/s); B 1, H 24 / 8, T 8191, D 128: 485 -> 328 us;
-// B 4, H 32 / 4, T 2048, D 64: 137 -> 121 us; B 8, H 12, T 1024, D 64: 43 -> 38 us; one tile (T 61): 10 us both.
+// (16 a clock and SM); at head_dim 64 512 against 1024.  At head_dim 128 and T 8191 both units run at about 66 %
+// of a CTA's time (ncu): a tile's chain of loading, maximum, exponentials and its two products is what is left over.  (2^x on
+// the FMA pipe for a quarter of the scores changed nothing, for more of them it was slower.)  One query tile per CTA with P
+// through shared memory, two CTAs per SM (attention_fwd_tile.cuh, which short launches still take), makes P's round trip and
+// the wait for its product part of every tile's chain.  That kernel -> this one, launches repeated, SM clock under load beside it:
+//   B 8, H 32, T 4096, D 128        1484 ->  937 us in short bursts, 1572 (1837 MHz) -> 1092 us (1537 MHz) for seconds under
+//                                   the power cap (741 -> 1174 and 699 -> 1007 TFLOP/s)
+//   B 1, H 24 / 8, T 8191, D 128     466 ->  317 us, 502 (1792 MHz) -> 368 us (1575 MHz)
+//   B 4, H 32 / 4, T 2048, D 64      125 ->  105 us (1965 MHz)
+//   B 8, H 12, T 1024, D 64         32.9 -> 28.6 us (1965 MHz), 43 -> 36 us with a cold L2
 //
 // The reference has no attention kernel in use: its CPU path materialises softmax(QK^T s + mask) V
 // (crates/incin-backends/src/cpu/ops/shape_ops.rs:1245-1269) and CUDA reports SDPA as unsupported;
@@ -51,8 +58,8 @@ struct FaCfg {
   static constexpr int SMEM_BYTES = OFF_BAR + 256 + 1024;
   // tensor memory: S_w (P_w in its first 64 columns) at [128 w, 128 w + 128), O_w at 256 + D w
   static constexpr int TMEM_COLS = 512, COL_O = 256;
-  // columns of P_w after which the first products of O_w += P_w V are let go: 96 of 128 takes 5 % off head_dim 128 (B 1,
-  // H 24 / 8, T 8191: 351 -> 335 us) and 3 % off head_dim 64 (B 4, H 32 / 4, T 2048: 122 -> 118 us); 64 is no better
+  // columns of P_w after which the first products of O_w += P_w V are let go: against none of them 96 of 128 took 5 % off
+  // head_dim 128 (B 1, H 24 / 8, T 8191) and 3 % off head_dim 64 (B 4, H 32 / 4, T 2048); 64 is no better
   static constexpr int PART = 96;
   static_assert(SMEM_BYTES <= 227 * 1024, "shared-memory plan");
 };
@@ -186,8 +193,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int j = 1; j < n && ok; ++j) ok = load_kv(&tmK, j) && load_kv(&tmV, j);
     }
   } else if (warp == 1) {
-    // issuer: the whole warp walks the loop, one elected lane executes the tcgen05 instructions.  Products of one
-    // issuing thread run in order, so S_w(j+1) may follow O_w += P_w(j) V_j directly although it overwrites P_w.
+    // issuer: the whole warp walks the loop, one elected lane executes the tcgen05 instructions.  S_w(j+1) follows
+    // O_w += P_w(j) V_j directly although it overwrites P_w: products of one issuing thread run in order.  (PTX states that
+    // for products of one accumulator and shape; for these two it is what the published kernels of this schedule rely on,
+    // and tests/test_attention_edges_gpu.py repeats the forward pass to the bit to catch an exception.)
     const bool leader = elect_one() != 0;
     constexpr uint32_t idesc_s = make_idesc_bf16(FA_BM, FA_BM, false, false);
     constexpr uint32_t idesc_o = make_idesc_bf16(FA_BM, D, false, true);
@@ -476,7 +485,11 @@ static int launch_fwd(const incin_attn_desc* d, cudaStream_t stream) {
   p.lse = d->lse;
   p.Tpad = n_q_tiles * FA_BM;
   p.status = (int*)d->status;
-  // K and V of every (batch, kv head) against half of the 126 MB L2
+  // K and V of every (batch, KV head) within 48 MB, about 40 % of L2: the line measured for the kernel with one tile per CTA
+  // (heaviest tiles first cost it 19 % at 512 MB).  For this one, all heads' heaviest pairs first | head by head, us: 24 MB
+  // (B 8, H 12, T 1024, D 64) 28.6 | 33.9, 32 MB (B 1, H 24 / 8, T 8191, D 128) 315 | 428, 96 MB (H 24) 335 | 441, 128 MB
+  // (B 2, H 32, T 4096) 250 | 265, 192 MB (B 6, H 24 / 8, T 8191) 2055 | 1983, 256 MB (B 8, H 32, T 2048) 297 | 277, 512 MB
+  // (T 4096) 1102 | 931: it lies nearer to 128 MB.
   p.pair_major = ((long long)d->B * d->Hkv * d->T * D * 2 * 2 <= (48ll << 20)) ? 1 : 0;
   const long long items = (long long)p.n_pairs * d->Hq * d->B;
   if (items > (1ll << 30)) return INCIN_ERR_TOO_LARGE;   // the kernel counts items in 32 bits

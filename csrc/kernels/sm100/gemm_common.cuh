@@ -340,7 +340,7 @@ __device__ __forceinline__ void epilogue_chunk(const GemmKernelParams& p, const 
 // The same for fp16 and tf32 products: alpha, then a bias in the operands' own type (fp16 or fp32), then fp32 or fp16
 // stores, 32 / 16 bytes at a time where the address allows.  A function of its own so that the bf16 epilogue keeps its
 // registers.  Writing the final type here replaced an fp32 result, a bias pass and a conversion pass (fp16, 4096 rows,
-// 768 -> 3072, forward + backward, with the backward's operands read as they lie: 288 -> 168 us a pass).
+// 768 -> 3072, forward + backward, with the backward's operands read as they lie: 281 -> 163 us a pass).
 __device__ __forceinline__ void epilogue_chunk_other(const GemmKernelParams& p, const uint32_t (&r)[32], void* c_ptr,
                                                      long long cbase, int nc, float alpha) {
   float v[32];

@@ -106,12 +106,12 @@ class _LinearF32Acc(torch.autograd.Function):
     """Linear for fp16 tensors and, under ``MathMode.FAST``, fp32 tensors (multiplied as tf32) on the same tcgen05
     kernel as the bf16 path: fp32 accumulation, bias in the epilogue, rounded once to the input type.  Gradients return
     through autograd.  The tensor cores read 16-bit operands of the backward products as they lie; tf32 operands have to
-    run along the reduction, so those are transposed first, the output gradient together with its column sums.  Sums have a fixed order, but for the fp32 weight gradient,
-    whose order is only fixed under ``Determinism.REQUIRED``.
+    run along the reduction, so those are transposed first, the output gradient together with its column sums.  Sums have a
+    fixed order, but for the fp32 weight gradient, whose order is only fixed under ``Determinism.REQUIRED``.
 
-    fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 288 -> 168 us and
-    271 -> 183 us a pass against products in fp32 with separate bias, conversion and transposition passes (both bound by
-    the host now; 80 us on the device for fp16)."""
+    fp16, 4096 rows, 768 -> 3072, and fp32, 8184 rows, 1024 -> 1000, forward + backward: 281 -> 163 us and
+    273 -> 185 us a pass against products in fp32 with separate bias, conversion and transposition passes (both bound by
+    the host now; 77 and 139 us on the device)."""
 
     @staticmethod
     def forward(ctx, x, w, b):
