@@ -155,6 +155,8 @@ class _LinearF32Acc(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             if half and n_out % unit == 0:
                 dw = torch.empty(n_out, n_in, dtype=w.dtype, device=dy.device)
+                if want_db:
+                    db = K.colsum(dy2, room=dw)
                 G.gemm(dy2, x2, dw, M=n_out, N=n_in, K=rows, lda=n_out, ldb=n_in, ldc=n_in, a_mn=True, b_mn=True)
             elif rows % unit:
                 dw = dy2.t() @ x2

@@ -154,13 +154,17 @@ def colsum_accum(dy, dbias):
               "colsum")
 
 
-def colsum(dy):
-    """Column sums of ``dy [..., N]`` in its own type: fp32 inside, one rounding, the same bits every time."""
+def colsum(dy, room=None):
+    """Column sums of ``dy [..., N]`` in its own type: fp32 inside, one rounding, the same bits every time.  ``room``: a
+    dense tensor that the next launch on this stream overwrites; its memory holds the partial sums where it is large enough."""
     N = dy.shape[-1]
     rows = dy.numel() // N
     lib = nat.cuda()
     out = torch.empty(N, dtype=dy.dtype, device=dy.device)
-    part = torch.empty(lib.incin_colsum_scratch_floats(rows, N), dtype=F32, device=dy.device)
+    floats = lib.incin_colsum_scratch_floats(rows, N)
+    part = room
+    if room is None or room.numel() * room.element_size() < 4 * floats:
+        part = torch.empty(floats, dtype=F32, device=dy.device)
     nat.check(lib.incin_colsum_typed(dy.data_ptr(), out.data_ptr(), part.data_ptr(), rows, N, N, _COLSUM_KIND[dy.dtype], _s()),
               "colsum")
     return out
