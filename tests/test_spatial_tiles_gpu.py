@@ -105,3 +105,20 @@ def test_strided_copy_merged_axes(shape, perm):
         assert torch.equal(T.materialize(t.permute(perm)), t.permute(perm).contiguous())
     wide = x[:, :, :, None].expand(*shape[:3], 3, shape[3])
     assert torch.equal(T.materialize(wide), wide.contiguous())
+
+
+def test_more_than_two_to_the_31_elements():
+    """Flat indexes of 64 bits: windows and cells of one element, so that every result is a copy of its input."""
+    from incin_b200.ops import tensor_ops as T
+    shape = (1, 3, 26755, 26756)
+    x = torch.empty(shape, dtype=torch.bfloat16, device="cuda").random_(-100, 100)
+    assert x.numel() > 2 ** 31
+    for op in (lambda t: T.max_pool2d(t, 1), lambda t: T.adaptive_avg_pool2d(t, shape[2:])):
+        leaf = x.detach().requires_grad_()
+        y = op(leaf)
+        assert torch.equal(y, x)
+        assert torch.equal(torch.autograd.grad(y, leaf, x)[0], x)
+        del y, leaf
+    cols = T.im2col(x, (1, 1))                  # K = 3: the general kernels
+    assert torch.equal(cols.view(*shape[2:], 3), x[0].permute(1, 2, 0))
+    assert torch.equal(T.col2im(cols, shape, (1, 1)), x)
